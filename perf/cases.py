@@ -300,8 +300,9 @@ def tolerance(case):
 
     Measured over the listed and forty drawn cases: attention on an f32 cache 3e-7; a step on one 3e-6, up to 9e-6
     (activations go to the matmuls as a high and a low bf16 part, 16 bits of mantissa); f32 queries on a bf16 cache
-    (both operands in two parts) and a step on one up to 3e-5 (a new key or value may round to the other neighbour); attention on an f16 cache 2.8e-4 (queries and
-    probabilities are f16), of which a step's logits show 8e-5; rows written as bf16 1.7e-3."""
+    (both operands in two parts) and a step on one up to 3e-5 (a new key or value may round to the other neighbour);
+    attention on an f16 cache 2.8e-4 (queries and probabilities are f16), of which a step's logits show 8e-5; rows
+    written as bf16 1.7e-3."""
     if case["kind"] == "step":
         return {"rel": {"f32": 4e-5, "bf16": 1.2e-4, "f16": 3.5e-4}[case["cache"]]}
     if case["halves"] and case["q"] == "bf16":
