@@ -548,6 +548,8 @@ void yx_ctx_destroy(yx_ctx *ctx) {
     if (ctx->lt_workspace) cudaFree(ctx->lt_workspace);
     release_matmul_library(ctx);
     if (ctx->idx_dev) cudaFree(ctx->idx_dev);
+    if (ctx->pick_counters) cudaFree(ctx->pick_counters);
+    if (ctx->pick_host) cudaFreeHost(ctx->pick_host);
     if (ctx->gather_buf) cudaFree(ctx->gather_buf);
     if (ctx->dev_status) cudaFreeHost(ctx->dev_status);
     for (auto &e : ctx->prof_events)

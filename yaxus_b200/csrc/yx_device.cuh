@@ -175,6 +175,14 @@ __device__ __forceinline__ float fast_exp2(float x) {
     return y;
 }
 
+// Where a kernel launched with launch_dependent (below) begins: everything earlier on the stream is
+// complete and visible after the wait, and only then may the kernel behind become resident in turn.
+// In that order a kernel that starts early knows that all kernels but the one just ahead are done.
+__device__ __forceinline__ void dependent_entry() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 __device__ __forceinline__ unsigned long long gtime() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -182,4 +190,24 @@ __device__ __forceinline__ unsigned long long gtime() {
 }
 
 }  // namespace dev
+
+// Launches a kernel as a programmatic dependent of the one ahead of it on the context's stream: it is
+// set up while that one still runs, which takes the launch latency and the drain between two small
+// kernels (2 to 3 us) out of the chain of a decode step.  The kernel begins with
+// griddepcontrol.wait (dev::dependent_entry, or later where it has work that needs no wait).
+template <typename... P, typename... A>
+int launch_dependent(yx_ctx *ctx, const char *what, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    ctx->launches++;
+    return check_cuda(ctx, cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...), what);
+}
 }  // namespace yx

@@ -344,8 +344,11 @@ struct yx_ctx {
     void *lt_handle = nullptr;             // cublasLtHandle_t, made at the first matmul of many rows
     void *lt_workspace = nullptr;
     size_t lt_workspace_cap = 0;
-    uint32_t *idx_dev = nullptr;           // token ids / row indices / argmax results of the model operators
+    uint32_t *idx_dev = nullptr;           // token ids / row indices / argmax parts of the model operators
     size_t idx_cap = 0;
+    uint32_t *pick_counters = nullptr;     // argmax: arrivals per row, zero between launches
+    uint32_t *pick_host = nullptr;         // argmax: the result, pinned and mapped
+    size_t pick_cap = 0;                   // rows both are made for
 
     // multi-GPU
     ncclComm *comm = nullptr;
