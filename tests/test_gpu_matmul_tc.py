@@ -1,0 +1,65 @@
+"""The many-row matmul at the edges of its tiles: ragged weight rows and pass rows, one and two tiles of
+pass rows, tiles shared along k by several CTA pairs, whole rounds before and after them."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+# x = hi + lo drops at most 2^-17 of each term (half a unit of lo's last place, against hi); the f32 sums
+# of 2 K terms err by a few 2^-24 of the terms' magnitudes.
+TOL = 2.0 ** -17 + 32 * 2.0 ** -24
+
+
+def dev(backend, x):
+    return torch.from_numpy(np.ascontiguousarray(x, np.float32)).to(backend.device)
+
+
+def magnitudes(x, w_bits):
+    """The sum of every product's terms' magnitudes."""
+    return np.abs(x.astype(np.float64)) @ np.abs((w_bits.astype(np.uint32) << 16).view(np.float32).astype(np.float64)).T
+
+
+def inputs(oracle, t, n, k):
+    rng = np.random.default_rng(t * 7919 + n + k)
+    x = rng.standard_normal((t, k)).astype(np.float32)
+    return x, oracle.to_bf16((rng.standard_normal((n, k)) / np.sqrt(k)).astype(np.float32))
+
+
+@pytest.mark.parametrize("t,n,k", [
+    (33, 1, 128), (64, 255, 128), (65, 257, 384), (256, 256, 1024), (257, 300, 640),   # fewer tiles than pairs
+    (40, 19300, 128), (300, 9700, 256),                                                # rounds and a remainder
+    (513, 6400, 128), (34, 18944, 128)])                                               # (the last: whole rounds where 74 pairs fit)
+def test_matmul_tiles(backend, oracle, t, n, k):
+    x, w_bits = inputs(oracle, t, n, k)
+    w, ref = backend.load_weight(w_bits), oracle.matmul(x, w_bits)
+    xd = dev(backend, x)
+    first = backend.to_host(backend.matmul(xd, w))
+    assert (np.abs(first - ref) <= TOL * magnitudes(x, w_bits)).all()
+    # the arrival counters are left clean, and shares are added up in one order
+    assert np.array_equal(backend.to_host(backend.matmul(xd, w)), first)
+
+
+@pytest.mark.parametrize("t,inner,k", [(33, 16, 128), (48, 144, 1024), (257, 1040, 256), (100, 24, 256), (35, 9696, 128)])
+def test_glu_tiles(backend, oracle, t, inner, k):
+    x, w_bits = inputs(oracle, t, 2 * inner, k)
+    w = backend.load_weight(w_bits)
+    xd = dev(backend, x)
+    got = backend.to_host(backend.matmul_glu(xd, w))
+    # silu(g) u moves by at most 1.1 |u| dg + |g| du: each product errs by TOL times its terms' magnitudes
+    s = oracle.matmul(x, w_bits)
+    mag = magnitudes(x, w_bits)
+    g, u = np.abs(s[:, :inner]), np.abs(s[:, inner:])
+    bound = TOL * (1.1 * u * mag[:, :inner] + g * mag[:, inner:]) + 1e-6 * np.maximum(1.0, g * u)
+    assert (np.abs(got - oracle.swiglu(s)) <= bound).all()
+    assert np.array_equal(backend.to_host(backend.matmul_glu(xd, w)), got)
+
+
+def test_unaligned_rows(backend, oracle):
+    # pass rows that start 8 bytes past a 16-byte boundary
+    x, w_bits = inputs(oracle, 70, 200, 256)
+    store = torch.zeros(70 * 256 + 2, dtype=torch.float32, device=backend.device)
+    xd = store[2:].view(70, 256)
+    xd.copy_(torch.from_numpy(x))
+    got = backend.to_host(backend.matmul(xd, backend.load_weight(w_bits)))
+    assert (np.abs(got - oracle.matmul(x, w_bits)) <= TOL * magnitudes(x, w_bits)).all()

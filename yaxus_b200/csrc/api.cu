@@ -117,8 +117,9 @@ int fold_device_status(yx_ctx *ctx) {
         yx_dev_status s = *ctx->dev_status;
         ctx->dev_status->code = 0;
         ctx->dev_status->expired = 0;
-        // A kernel that gave up may have left arrival counters of the fused merge non-zero.
+        // A kernel that gave up may have left arrival counters (fused merge, shared matmul tiles) non-zero.
         if (ctx->counters) cudaMemsetAsync(ctx->counters, 0, ctx->counters_cap, ctx->stream);
+        if (ctx->mm_counters) cudaMemsetAsync(ctx->mm_counters, 0, ctx->mm_counters_cap, ctx->stream);
         return fail(ctx, YX_ERR_DEVICE,
                     "a kernel reported a failed check: code " + std::to_string(s.code) + " at " +
                         std::to_string(s.where) + " (" + std::to_string(s.a) + ", " + std::to_string(s.b) + ")" +
@@ -545,8 +546,8 @@ void yx_ctx_destroy(yx_ctx *ctx) {
     if (ctx->counters) cudaFree(ctx->counters);
     if (ctx->mm_part) cudaFree(ctx->mm_part);
     if (ctx->mm_packed) cudaFree(ctx->mm_packed);
-    if (ctx->lt_workspace) cudaFree(ctx->lt_workspace);
-    release_matmul_library(ctx);
+    if (ctx->mm_sums) cudaFree(ctx->mm_sums);
+    if (ctx->mm_counters) cudaFree(ctx->mm_counters);
     if (ctx->idx_dev) cudaFree(ctx->idx_dev);
     if (ctx->pick_counters) cudaFree(ctx->pick_counters);
     if (ctx->pick_host) cudaFreeHost(ctx->pick_host);

@@ -1,0 +1,502 @@
+// out [T, N] f32 = x [T, K] f32 . w [N, K]^T (bf16) for passes of many rows, on the fifth-generation
+// tensor cores, and the same with silu(gate) * up taken in the epilogue (crates/yaxus-model/src/lib.rs:128,164-168).
+//
+// Activations keep 16 bits of mantissa: x = hi + lo, two bf16 matrices, and every weight tile that reaches
+// shared memory is multiplied by both, into one f32 accumulator in tensor memory.  The arithmetic is twice
+// that of a plain bf16 product; what a tile costs in weight traffic, accumulator reads and stores is not.
+//
+// The products are taken transposed, out^T = w x^T, by pairs of CTAs (cta_group::2): a tile is 256 weight
+// rows (128 in each CTA) by up to 256 pass rows (half of them in each CTA), so a lane of tensor memory is a
+// weight row, a warp's store of one pass row is one 128-byte line, and a pass of 33 rows fills the 256-row
+// side as well as one of 2048 does.  A k step of 64 costs a CTA 16 KiB of weights and up to 32 KiB of
+// activations for 2 x 256 x 256 x 64 multiply-adds: 32 bytes a clock and SM, half of what L2 delivers.
+//
+// Tiles are dealt to the pairs in whole rounds, pass rows fastest, so that the pairs that run together share
+// weight rows and activations in L2.  What is left after the last whole round is cut along k into one equal
+// share a pair (stream-K): such a share's sums go to scratch, and the CTA that comes last at a tile adds them
+// up in order.  The shares come first in a pair's work, so that the adding up hides under whole tiles.  Adding up
+// is a chain of L2 latencies: with one warp to a lane quarter and one share at a time it took 15 to 20 us.
+//
+// Large passes are bound by the tensor cores: 2048 rows on 4096 -> 28672 (gate and up) take 625 us, 1.54 PFLOP/s
+// of bf16 products; 80 rows by the weights' way through L2 and shared memory: 412 MB in 100 us.  Against two
+// library products (high part, then low part added to it) and a SwiGLU kernel, whole steps of one layer went from
+// 2151 to 1776 us (2048 rows) and from 1244 to 387 us (80 rows).
+//
+// Warps 0-7 epilogue (two to each 32 lanes of tensor memory, taking turns at 32 pass rows), warp 8 TMA, warp 9
+// issues the MMAs (first CTA of the pair).  All waits are bounded; on expiry the CTA records where, stops waiting anywhere, frees its
+// tensor memory together with its partner and returns.
+#include <cuda.h>
+
+#include <algorithm>
+
+#include "yx_tcgen05.cuh"
+
+namespace yx {
+namespace {
+
+using namespace dev;
+
+constexpr uint32_t TC_M = 256;              // weight rows of a pair's tile
+constexpr uint32_t TC_KSTEP = 64;           // k of a stage: one 128-byte swizzled row
+constexpr uint32_t TC_MAX_BT = 256;         // pass rows of a tile
+constexpr int TC_MAX_STAGES = 12;
+constexpr int TC_THREADS = 10 * 32;
+constexpr int TC_TMA_WARP = 8, TC_MMA_WARP = 9;
+constexpr uint32_t W_BYTES = 128 * 128;     // a CTA's share of a stage's weights
+constexpr uint32_t TC_SMEM_BUDGET = 220 * 1024;
+constexpr uint32_t GLU_GROUP = 16;          // gate and up rows alternate in a tile sixteen by sixteen: a warp holds both
+
+struct PairArgs {
+    uint32_t T, cols;                 // pass rows; columns of the result
+    uint32_t bt, t_tiles;             // pass rows of a tile (multiple of 32), tiles of them
+    uint32_t ksteps;
+    uint32_t pairs;                   // CTA pairs of the grid
+    uint32_t rounds;                  // whole rounds of tiles
+    uint32_t rest_units, rest_pairs;  // k steps of the tiles after them, and the pairs that share those
+    uint32_t stages;
+    float *out;
+    float *part;                      // [2 * rest_pairs shares][2 CTAs][bt][128]
+    uint32_t *counters;               // [tiles left over][2 CTAs], zero between launches
+    yx_dev_status *status;
+};
+
+// One stretch of k steps of one tile.
+struct Piece {
+    uint32_t tile, k0, k1;
+    bool whole;
+};
+
+__device__ __forceinline__ uint32_t rest_begin(const PairArgs &a, uint32_t p) { return (uint32_t)((uint64_t)p * a.rest_units / a.rest_pairs); }
+// The pair whose share holds unit u.
+__device__ __forceinline__ uint32_t rest_owner(const PairArgs &a, uint32_t u) {
+    return (uint32_t)((((uint64_t)u + 1) * a.rest_pairs - 1) / a.rest_units);
+}
+
+// Walks a pair's pieces: its share of the left-over tiles (at most two pieces), then its whole tiles.
+struct Walk {
+    uint32_t u, u_end, round;
+    __device__ __forceinline__ Walk(const PairArgs &a, uint32_t pair) : u(0), u_end(0), round(0) {
+        if (pair < a.rest_pairs) {
+            u = rest_begin(a, pair);
+            u_end = rest_begin(a, pair + 1);
+        }
+    }
+    __device__ __forceinline__ bool next(const PairArgs &a, uint32_t pair, Piece &p) {
+        if (u < u_end) {
+            const uint32_t tile = u / a.ksteps;
+            p.k0 = u - tile * a.ksteps;
+            p.k1 = min(a.ksteps, p.k0 + (u_end - u));
+            u += p.k1 - p.k0;
+            p.tile = a.rounds * a.pairs + tile;
+            p.whole = p.k1 - p.k0 == a.ksteps;
+            return true;
+        }
+        if (round >= a.rounds) return false;
+        p = Piece{round * a.pairs + pair, 0, a.ksteps, true};
+        round++;
+        return true;
+    }
+};
+
+__device__ __forceinline__ uint32_t mapa(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// 32 pass rows from `t0` on of this lane's weight row.
+template <bool GLU>
+__device__ __forceinline__ void store_rows(const PairArgs &a, const float (&v)[32], uint32_t t0, uint32_t row, int lane) {
+    if constexpr (!GLU) {
+        if (row >= a.cols) return;
+        float *dst = a.out + (size_t)t0 * a.cols + row;
+        if (t0 + 32 <= a.T) {
+#pragma unroll
+            for (int i = 0; i < 32; i++) dst[(size_t)i * a.cols] = v[i];
+        } else {
+#pragma unroll
+            for (int i = 0; i < 32; i++)
+                if (t0 + i < a.T) dst[(size_t)i * a.cols] = v[i];
+        }
+    } else {
+        // Lanes 0-15 hold gate rows, lanes 16-31 the same rows' up: the lower half finishes the first sixteen
+        // pass rows, the upper half the others.  `row` counts both kinds, so its 32 are 16 columns.
+        const uint32_t col = (row >> 5) * GLU_GROUP + (lane & 15), t = t0 + (lane & 16);
+        float *dst = a.out + (size_t)t * a.cols + col;
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+            const float other = __shfl_xor_sync(0xffffffffu, lane < 16 ? v[16 + i] : v[i], 16);
+            const float g = lane < 16 ? v[i] : other, u = lane < 16 ? other : v[16 + i];
+            if (col < a.cols && t + i < a.T) dst[(size_t)i * a.cols] = g / (1.0f + expf(-g)) * u;
+        }
+    }
+}
+
+template <bool GLU>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
+matmul_pair_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap x_map, const PairArgs a) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    __shared__ __align__(8) uint64_t bar_store[2 * TC_MAX_STAGES + 4];
+    __shared__ uint32_t tmem_base_s;
+    __shared__ int abort_flag;
+    __shared__ int last_s;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = blockIdx.x & 1u, pair = blockIdx.x >> 1;
+    const uint32_t S = a.stages, x_bytes = a.bt * 128u, stage_bytes = W_BYTES + x_bytes;   // x: bt / 2 rows, high and low part
+    const uint32_t base = smem_u32(smem);
+    const uint32_t b_full = smem_u32(bar_store), b_empty = b_full + 8 * TC_MAX_STAGES;
+    const uint32_t b_acc_full = b_empty + 8 * TC_MAX_STAGES, b_acc_empty = b_acc_full + 16;
+    volatile int *abortp = &abort_flag;
+
+    if (threadIdx.x == 0) {
+        abort_flag = 0;
+        for (uint32_t s = 0; s < S; s++) {
+            mbar_init(b_full + 8 * s, 1);
+            mbar_init(b_empty + 8 * s, 1);
+        }
+        for (int b = 0; b < 2; b++) {
+            mbar_init(b_acc_full + 8 * b, 1);
+            mbar_init(b_acc_empty + 8 * b, 16);   // a warp's arrival each, from both CTAs
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == TC_TMA_WARP && lane == 0) {
+        prefetch_tensormap(&w_map);
+        prefetch_tensormap(&x_map);
+    }
+    if (warp == TC_MMA_WARP) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)), "n"(512) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();
+    tc_fence_after();
+    const uint32_t tmem = tmem_base_s;
+
+    if (warp == TC_TMA_WARP && lane == 0) {
+        // ---- producer -------------------------------------------------------------------------
+        const uint32_t full0 = mapa(b_full, 0);   // the first CTA's barriers count both CTAs' bytes
+        auto load_w = [&](uint32_t s, const Piece &p, uint32_t k) {
+            const uint32_t m0 = (p.tile / a.t_tiles) * TC_M + rank * 128u;
+            if (rank == 0) mbar_expect_tx(b_full + 8 * s, 2 * stage_bytes);
+            tma_load_4d_pair(base + s * stage_bytes, &w_map, (int)(k * TC_KSTEP), GLU ? 0 : (int)m0, 0, GLU ? (int)(m0 / (2 * GLU_GROUP)) : 0,
+                             full0 + 8 * s);
+        };
+        auto load_x = [&](uint32_t s, const Piece &p, uint32_t k) {
+            const uint32_t t0 = (p.tile % a.t_tiles) * a.bt + rank * (a.bt / 2);
+            tma_load_3d_pair(base + s * stage_bytes + W_BYTES, &x_map, (int)(k * TC_KSTEP), (int)t0, 0, full0 + 8 * s);
+        };
+        // The kernel ahead (the split of the activations) let this one start only after its own wait, so nothing
+        // that may still run writes the weights: the ring's first weights are on their way before the wait.
+        uint32_t ahead = 0;
+        {
+            Walk walk(a, pair);
+            Piece p;
+            while (ahead < S && walk.next(a, pair, p))
+                for (uint32_t k = p.k0; k < p.k1 && ahead < S; k++) load_w(ahead++, p, k);
+        }
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        Walk walk(a, pair);
+        Piece p;
+        uint32_t it = 0, s = 0, phase = 0;
+        while (walk.next(a, pair, p)) {
+            for (uint32_t k = p.k0; k < p.k1; k++, it++) {
+                if (it >= ahead) {
+                    mbar_wait(b_empty + 8 * s, phase ^ 1u, abortp, a.status, 501);
+                    if (*abortp) break;
+                    load_w(s, p, k);
+                }
+                load_x(s, p, k);
+                if (++s == S) {
+                    s = 0;
+                    phase ^= 1u;
+                }
+            }
+            if (*abortp) break;
+        }
+    } else if (warp == TC_MMA_WARP && lane == 0 && rank == 0) {
+        // ---- MMA issuer -----------------------------------------------------------------------
+        const uint32_t idesc = f16_instr_desc(true, false, TC_M, a.bt);
+        Walk walk(a, pair);
+        Piece p;
+        uint32_t s = 0, phase = 0;
+        for (uint32_t n = 0; walk.next(a, pair, p) && !*abortp; n++) {
+            const uint32_t buf = n & 1u, acc = tmem + buf * TC_MAX_BT;
+            if (n >= 2) mbar_wait(b_acc_empty + 8 * buf, ((n >> 1) - 1) & 1u, abortp, a.status, 502);
+            tc_fence_after();
+            for (uint32_t k = p.k0; k < p.k1; k++) {
+                mbar_wait(b_full + 8 * s, phase, abortp, a.status, 503);
+                if (*abortp) break;
+                tc_fence_after();
+                const uint32_t w_lo = desc_lo(base + s * stage_bytes, 0), h_lo = w_lo + W_BYTES / 16, l_lo = h_lo + x_bytes / 32;
+#pragma unroll
+                for (uint32_t kk = 0; kk < 4; kk++) umma2_ss_lo(acc, w_lo + 2 * kk, h_lo + 2 * kk, idesc, k > p.k0 || kk > 0);
+#pragma unroll
+                for (uint32_t kk = 0; kk < 4; kk++) umma2_ss_lo(acc, w_lo + 2 * kk, l_lo + 2 * kk, idesc, 1);
+                umma2_commit(b_empty + 8 * s);
+                if (++s == S) {
+                    s = 0;
+                    phase ^= 1u;
+                }
+            }
+            umma2_commit(b_acc_full + 8 * buf);
+        }
+    } else if (warp < 8) {
+        // ---- epilogue -------------------------------------------------------------------------
+        Walk walk(a, pair);
+        Piece p;
+        for (uint32_t n = 0; walk.next(a, pair, p); n++) {
+            const uint32_t buf = n & 1u, acc = tmem + buf * TC_MAX_BT + ((uint32_t)(warp & 3) << 21);
+            const uint32_t wr = (warp & 3) * 32 + lane;   // weight row of this CTA's 128
+            const uint32_t row = (p.tile / a.t_tiles) * TC_M + rank * 128u + wr, t0 = (p.tile % a.t_tiles) * a.bt;
+            mbar_wait(b_acc_full + 8 * buf, (n >> 1) & 1u, abortp, a.status, 504);
+            __syncwarp();   // (after a wait that ran out the warps go on, on whatever is there: their barriers below count all of them)
+            tc_fence_after();
+            const uint32_t rest = p.whole ? 0u : p.tile - a.rounds * a.pairs;
+            // The pairs that share left-over tile `rest`.  Only the first of them may have begun in the tile before it,
+            // which makes this tile its second piece.
+            uint32_t q0 = 0, q1 = 0, second = 0;
+            if (!p.whole) {
+                q0 = rest_owner(a, rest * a.ksteps);
+                q1 = rest_owner(a, (rest + 1) * a.ksteps - 1);
+                second = rest - rest_begin(a, q0) / a.ksteps;
+            }
+            // A share's sums: four pass rows of each of 128 weight rows, then the next four.
+            auto share = [&](uint32_t q) { return (float4 *)(a.part + ((size_t)(2 * q + (q == q0 ? second : 0u)) * 2 + rank) * a.bt * 128u) + wr; };
+            for (uint32_t c = 32u * (warp >> 2); c < a.bt; c += 64) {
+                uint32_t r[32];
+                tmem_ld32(acc + c, r);
+                tmem_ld_wait();
+                if (p.whole) {
+                    float v[32];
+#pragma unroll
+                    for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
+                    store_rows<GLU>(a, v, t0 + c, row, lane);
+                } else {
+                    float4 *mine = share(pair) + c / 4 * 128u;
+#pragma unroll
+                    for (int i = 0; i < 8; i++)
+                        __stcg(mine + i * 128, make_float4(__uint_as_float(r[4 * i]), __uint_as_float(r[4 * i + 1]), __uint_as_float(r[4 * i + 2]),
+                                                           __uint_as_float(r[4 * i + 3])));
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0)
+                asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(mapa(b_acc_empty + 8 * buf, 0)) : "memory");
+            if (p.whole) continue;
+            // The last of the tile's shares to arrive adds all of them up, in the order of k.
+            __threadfence();
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+            if (threadIdx.x == 0) {
+                uint32_t *counter = a.counters + 2 * rest + rank;
+                const int last = atomicAdd(counter, 1u) == q1 - q0;
+                if (last) *counter = 0u;
+                last_s = last;
+            }
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+            const bool last = last_s != 0;
+            if (!last) continue;
+            __threadfence();
+            // (a chain of L2 latencies: six shares' sums are asked for at once)
+            for (uint32_t c = 32u * (warp >> 2); c < a.bt && t0 + c < a.T; c += 64) {
+                alignas(16) float v[32];
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    float4 sum[4] = {};
+                    for (uint32_t q = q0; q <= q1; q += 6) {
+                        float4 w[6][4];
+#pragma unroll
+                        for (int b = 0; b < 6; b++) {
+                            const float4 *src = share(min(q + b, q1)) + (c / 4 + 4 * h) * 128u;
+#pragma unroll
+                            for (int i = 0; i < 4; i++) w[b][i] = q + b <= q1 ? __ldcg(src + i * 128) : make_float4(0.f, 0.f, 0.f, 0.f);
+                        }
+#pragma unroll
+                        for (int b = 0; b < 6; b++)
+#pragma unroll
+                            for (int i = 0; i < 4; i++) {
+                                sum[i].x += w[b][i].x;
+                                sum[i].y += w[b][i].y;
+                                sum[i].z += w[b][i].z;
+                                sum[i].w += w[b][i].w;
+                            }
+                    }
+#pragma unroll
+                    for (int i = 0; i < 4; i++) *(float4 *)(v + 16 * h + 4 * i) = sum[i];
+                }
+                store_rows<GLU>(a, v, t0 + c, row, lane);
+            }
+        }
+    }
+    __syncwarp();
+    if (*abortp)
+        for (int i = 0; i < 64; i++) __nanosleep(1000);   // copies and products in flight come to rest
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();   // the partner's copies and completions still land in this CTA
+    tc_fence_after();
+    if (warp == TC_MMA_WARP) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(512) : "memory");
+}
+
+// x [n] f32 -> its high and its low bf16 part, x = hi + lo to 16 bits of mantissa; eight elements a thread.
+template <bool VEC16>
+__global__ void __launch_bounds__(256) split_rows_kernel(const float *__restrict__ x, size_t n, uint4 *__restrict__ hi, uint4 *__restrict__ lo) {
+    dependent_entry();
+    const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx * 8 >= n) return;
+    float v[8];
+    if constexpr (VEC16) {
+        *(float4 *)v = *(const float4 *)(x + idx * 8);
+        *(float4 *)(v + 4) = *(const float4 *)(x + idx * 8 + 4);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; j++) *(float2 *)(v + 2 * j) = *(const float2 *)(x + idx * 8 + 2 * j);
+    }
+    uint32_t h[4], l[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        h[j] = pack2<true>(v[2 * j], v[2 * j + 1]);
+        const float2 b = unpack2<true>(h[j]);
+        l[j] = pack2<true>(v[2 * j] - b.x, v[2 * j + 1] - b.y);
+    }
+    hi[idx] = make_uint4(h[0], h[1], h[2], h[3]);
+    lo[idx] = make_uint4(l[0], l[1], l[2], l[3]);
+}
+
+using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
+                                 const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiled encode_tiled() {
+    static const EncodeTiled fn = [] {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess)
+            p = nullptr;
+        return (EncodeTiled)p;
+    }();
+    return fn;
+}
+
+// A map of a bf16 tensor, innermost dimension dense, 128-byte swizzle; rows outside it read as zero.
+int encode(yx_ctx *ctx, CUtensorMap *map, uint32_t rank, const void *p, const cuuint64_t *dims, const cuuint64_t *strides, const cuuint32_t *box) {
+    const cuuint32_t ones[4] = {1, 1, 1, 1};
+    if (!encode_tiled()) return fail(ctx, YX_ERR_CUDA, "matmul: the driver has no cuTensorMapEncodeTiled");
+    const CUresult r = encode_tiled()(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<void *>(p), dims, strides, box, ones,
+                                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? YX_OK : fail(ctx, YX_ERR_CUDA, "matmul: cuTensorMapEncodeTiled failed with " + std::to_string((int)r));
+}
+
+// The weights in boxes of 128 rows by 64 k; for a GLU four groups of 16 gate rows and the 16 up rows of the same columns.
+int encode_weights(yx_ctx *ctx, CUtensorMap *map, const void *w, uint32_t N, uint32_t K, bool glu) {
+    const cuuint64_t row = (cuuint64_t)K * 2;
+    if (glu) {
+        const cuuint64_t dims[4] = {K, GLU_GROUP, 2, N / 2 / GLU_GROUP};
+        const cuuint64_t strides[3] = {row, N / 2 * row, GLU_GROUP * row};
+        const cuuint32_t box[4] = {TC_KSTEP, GLU_GROUP, 2, 128 / (2 * GLU_GROUP)};
+        return encode(ctx, map, 4, w, dims, strides, box);
+    }
+    const cuuint64_t dims[4] = {K, N, 1, 1};
+    const cuuint64_t strides[3] = {row, N * row, N * row};
+    const cuuint32_t box[4] = {TC_KSTEP, 128, 1, 1};
+    return encode(ctx, map, 4, w, dims, strides, box);
+}
+
+int ensure_counters(yx_ctx *ctx, size_t n) {
+    const size_t before = ctx->mm_counters_cap;
+    if (int rc = ensure_buffer(ctx, (void **)&ctx->mm_counters, &ctx->mm_counters_cap, std::max<size_t>(n, 512) * sizeof(uint32_t))) return rc;
+    if (ctx->mm_counters_cap == before) return YX_OK;
+    return check_cuda(ctx, cudaMemsetAsync(ctx->mm_counters, 0, ctx->mm_counters_cap, ctx->stream), "matmul: counters");
+}
+
+// CTA pairs that are on the chip together (a GPC with an odd number of SMs leaves one out).
+template <bool GLU>
+int resident_pairs(yx_ctx *ctx, int *out) {
+    int &n = ctx->mm_pairs[GLU];
+    if (n == 0) {
+        auto *kernel = matmul_pair_kernel<GLU>;
+        if (int rc = check_cuda(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_BUDGET),
+                                "matmul: shared memory attribute"))
+            return rc;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)ctx->sm_count / 2 * 2);
+        cfg.blockDim = dim3(TC_THREADS);
+        cfg.dynamicSmemBytes = TC_SMEM_BUDGET;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 2;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int found = 0;
+        if (int rc = check_cuda(ctx, cudaOccupancyMaxActiveClusters(&found, kernel, &cfg), "matmul: resident pairs")) return rc;
+        n = std::max(1, std::min(found, ctx->sm_count / 2));
+    }
+    *out = n;
+    return YX_OK;
+}
+
+template <bool GLU>
+int matmul_pair_rows(yx_ctx *ctx, const float *x, const void *w, uint32_t T, uint32_t N, uint32_t K, float *out) {
+    const size_t n = (size_t)T * K;
+    if (int rc = ensure_buffer(ctx, (void **)&ctx->mm_packed, &ctx->mm_packed_cap, n * 4)) return rc;
+    int pairs = 0;
+    if (int rc = resident_pairs<GLU>(ctx, &pairs)) return rc;
+
+    PairArgs a{};
+    a.T = T;
+    a.cols = GLU ? N / 2 : N;
+    // Pass rows are spread evenly over as few tiles as hold them: 300 rows are two tiles of 160, not 256 and 64.
+    a.t_tiles = (T + TC_MAX_BT - 1) / TC_MAX_BT;
+    a.bt = ((T + a.t_tiles - 1) / a.t_tiles + 31) / 32 * 32;
+    a.ksteps = K / TC_KSTEP;
+    const uint32_t tiles = ((N + TC_M - 1) / TC_M) * a.t_tiles;
+    a.pairs = (uint32_t)pairs;
+    a.rounds = tiles / a.pairs;
+    a.rest_units = (tiles - a.rounds * a.pairs) * a.ksteps;
+    // (a share of fewer than four k steps costs more to add up than it saves)
+    if (a.rest_units > 0) a.rest_pairs = std::min(a.pairs, std::max(1u, a.rest_units / std::min(4u, a.ksteps)));
+    const uint32_t stage_bytes = W_BYTES + a.bt * 128u;
+    a.stages = std::min<uint32_t>(TC_MAX_STAGES, (TC_SMEM_BUDGET - 1024) / stage_bytes);
+    a.out = out;
+    a.status = ctx->dev_status;
+    if (int rc = ensure_buffer(ctx, (void **)&ctx->mm_part, &ctx->mm_part_cap,
+                               std::max<size_t>((size_t)a.rest_pairs * 2 * 2 * a.bt * 128 * sizeof(float), 16)))
+        return rc;
+    a.part = ctx->mm_part;
+    if (int rc = ensure_counters(ctx, 2 * (tiles - a.rounds * a.pairs))) return rc;
+    a.counters = ctx->mm_counters;
+
+    CUtensorMap w_map, x_map;
+    if (int rc = encode_weights(ctx, &w_map, w, N, K, GLU)) return rc;
+    uint4 *hi = (uint4 *)ctx->mm_packed, *lo = hi + n / 8;
+    {
+        const cuuint64_t dims[3] = {K, T, 2};
+        const cuuint64_t strides[2] = {(cuuint64_t)K * 2, (cuuint64_t)T * K * 2};
+        const cuuint32_t box[3] = {TC_KSTEP, a.bt / 2, 2};
+        if (int rc = encode(ctx, &x_map, 3, hi, dims, strides, box)) return rc;
+    }
+    ctx->last_launch = yx_ctx::LAST_OTHER;
+    if (int rc = launch_dependent(ctx, "matmul: activation split kernel launch", ((uintptr_t)x & 15u) == 0 ? split_rows_kernel<true> : split_rows_kernel<false>,
+                                  dim3((unsigned)((n / 8 + 255) / 256)), dim3(256), 0, x, n, hi, lo))
+        return rc;
+    const uint32_t grid = 2 * (a.rounds > 0 ? a.pairs : a.rest_pairs);
+    return launch_dependent(ctx, "matmul kernel launch", matmul_pair_kernel<GLU>, dim3(grid), dim3(TC_THREADS), a.stages * stage_bytes, w_map, x_map, a);
+}
+
+}  // namespace
+
+// Takes K a multiple of 64, w 16-byte aligned, x 8-byte aligned; with `glu`, a multiple of 16 result columns.
+int launch_matmul_tc(yx_ctx *ctx, const float *x, const void *w, uint32_t T, uint32_t N, uint32_t K, bool glu, float *out) {
+    return glu ? matmul_pair_rows<true>(ctx, x, w, T, N, K, out) : matmul_pair_rows<false>(ctx, x, w, T, N, K, out);
+}
+
+}  // namespace yx

@@ -14,13 +14,8 @@
 // eight consecutive k of one weight row, which permutes k inside a step the same way for both
 // operands, so the products pair up correctly.
 //
-// Passes of more than 32 rows (prompt chunks) are a plain GEMM and go to cuBLASLt, loaded at run
-// time like NCCL; the activations' high and low bf16 parts are two GEMMs into one f32 result.
-// Without the library the row kernel takes the rows 32 at a time, streaming the weights again
-// for each block.
-#include <cublasLt.h>
+// Passes of more than 32 rows (prompt chunks, verification) go to the tcgen05 kernel of matmul_tc.cu.
 #include <cuda_bf16.h>
-#include <dlfcn.h>
 #include <string.h>
 
 #include <algorithm>
@@ -456,134 +451,6 @@ int launched(yx_ctx *ctx, const char *what) {
     return check_cuda(ctx, cudaGetLastError(), what);
 }
 
-// ---- cuBLASLt, for passes of many rows --------------------------------------------------------
-struct Lt {
-    void *lib = nullptr;
-    bool tried = false;
-    cublasStatus_t (*create)(cublasLtHandle_t *) = nullptr;
-    cublasStatus_t (*destroy)(cublasLtHandle_t) = nullptr;
-    cublasStatus_t (*desc_create)(cublasLtMatmulDesc_t *, cublasComputeType_t, cudaDataType_t) = nullptr;
-    cublasStatus_t (*desc_destroy)(cublasLtMatmulDesc_t) = nullptr;
-    cublasStatus_t (*desc_set)(cublasLtMatmulDesc_t, cublasLtMatmulDescAttributes_t, const void *, size_t) = nullptr;
-    cublasStatus_t (*layout_create)(cublasLtMatrixLayout_t *, cudaDataType_t, uint64_t, uint64_t, int64_t) = nullptr;
-    cublasStatus_t (*layout_destroy)(cublasLtMatrixLayout_t) = nullptr;
-    cublasStatus_t (*pref_create)(cublasLtMatmulPreference_t *) = nullptr;
-    cublasStatus_t (*pref_destroy)(cublasLtMatmulPreference_t) = nullptr;
-    cublasStatus_t (*pref_set)(cublasLtMatmulPreference_t, cublasLtMatmulPreferenceAttributes_t, const void *, size_t) = nullptr;
-    cublasStatus_t (*heuristic)(cublasLtHandle_t, cublasLtMatmulDesc_t, cublasLtMatrixLayout_t, cublasLtMatrixLayout_t,
-                                cublasLtMatrixLayout_t, cublasLtMatrixLayout_t, cublasLtMatmulPreference_t, int,
-                                cublasLtMatmulHeuristicResult_t *, int *) = nullptr;
-    cublasStatus_t (*matmul)(cublasLtHandle_t, cublasLtMatmulDesc_t, const void *, const void *, cublasLtMatrixLayout_t,
-                             const void *, cublasLtMatrixLayout_t, const void *, const void *, cublasLtMatrixLayout_t, void *,
-                             cublasLtMatrixLayout_t, const cublasLtMatmulAlgo_t *, void *, size_t, cudaStream_t) = nullptr;
-    bool ok() const { return matmul != nullptr; }
-};
-
-Lt load_lt() {
-    Lt l;
-    l.tried = true;
-    const char *names[] = {"libcublasLt.so.12", "libcublasLt.so", "/usr/local/cuda/lib64/libcublasLt.so.12"};
-    for (const char *n : names) {
-        l.lib = dlopen(n, RTLD_NOW | RTLD_GLOBAL);
-        if (l.lib) break;
-    }
-    if (!l.lib) return l;
-    auto sym = [&](const char *n) { return dlsym(l.lib, n); };
-    l.create = (decltype(l.create))sym("cublasLtCreate");
-    l.destroy = (decltype(l.destroy))sym("cublasLtDestroy");
-    l.desc_create = (decltype(l.desc_create))sym("cublasLtMatmulDescCreate");
-    l.desc_destroy = (decltype(l.desc_destroy))sym("cublasLtMatmulDescDestroy");
-    l.desc_set = (decltype(l.desc_set))sym("cublasLtMatmulDescSetAttribute");
-    l.layout_create = (decltype(l.layout_create))sym("cublasLtMatrixLayoutCreate");
-    l.layout_destroy = (decltype(l.layout_destroy))sym("cublasLtMatrixLayoutDestroy");
-    l.pref_create = (decltype(l.pref_create))sym("cublasLtMatmulPreferenceCreate");
-    l.pref_destroy = (decltype(l.pref_destroy))sym("cublasLtMatmulPreferenceDestroy");
-    l.pref_set = (decltype(l.pref_set))sym("cublasLtMatmulPreferenceSetAttribute");
-    l.heuristic = (decltype(l.heuristic))sym("cublasLtMatmulAlgoGetHeuristic");
-    auto mm = (decltype(l.matmul))sym("cublasLtMatmul");
-    if (l.create && l.destroy && l.desc_create && l.desc_destroy && l.desc_set && l.layout_create && l.layout_destroy &&
-        l.pref_create && l.pref_destroy && l.pref_set && l.heuristic)
-        l.matmul = mm;
-    return l;
-}
-
-// (initialised once, by whichever thread comes first)
-Lt &lt() {
-    static Lt l = load_lt();
-    return l;
-}
-
-// x [T][K] f32 -> hi [T][K] and lo [T][K] bf16, x = hi + lo to 16 bits of mantissa.
-__global__ void split_rows_kernel(const float *__restrict__ x, size_t n, __nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *__restrict__ lo) {
-    const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= n) return;
-    const float v = x[idx];
-    const __nv_bfloat16 h = __float2bfloat16_rn(v);
-    hi[idx] = h;
-    lo[idx] = __float2bfloat16_rn(v - __bfloat162float(h));
-}
-
-constexpr size_t LT_WORKSPACE = 32u << 20;
-
-// out [T][N] (row-major f32) = x . w^T through cuBLASLt.  In its column-major terms the result is
-// the N x T matrix w^T(K x N, transposed) times x^T (K x T).  Returns -1 when the library or a
-// kernel for the shape is not there (the caller then uses the row kernel), else a yx_error.
-int matmul_lt(yx_ctx *ctx, const float *x, const __nv_bfloat16 *w, uint32_t T, uint32_t N, uint32_t K, float *out) {
-    Lt &l = lt();
-    if (!l.ok()) return -1;
-    if (!ctx->lt_handle) {
-        cublasLtHandle_t h = nullptr;
-        if (l.create(&h) != CUBLAS_STATUS_SUCCESS) return -1;
-        ctx->lt_handle = h;
-    }
-    if (int rc = ensure_buffer(ctx, (void **)&ctx->mm_packed, &ctx->mm_packed_cap, (size_t)T * K * 4)) return rc;
-    if (int rc = ensure_buffer(ctx, (void **)&ctx->lt_workspace, &ctx->lt_workspace_cap, LT_WORKSPACE)) return rc;
-    __nv_bfloat16 *hi = (__nv_bfloat16 *)ctx->mm_packed, *lo = hi + (size_t)T * K;
-    const size_t n = (size_t)T * K;
-    split_rows_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(x, n, hi, lo);
-    if (int rc = launched(ctx, "matmul: activation split kernel")) return rc;
-
-    cublasLtMatmulDesc_t desc = nullptr;
-    cublasLtMatrixLayout_t la = nullptr, lb = nullptr, lc = nullptr;
-    cublasLtMatmulPreference_t pref = nullptr;
-    int result = -1;
-    do {
-        if (l.desc_create(&desc, CUBLAS_COMPUTE_32F, CUDA_R_32F) != CUBLAS_STATUS_SUCCESS) break;
-        const cublasOperation_t ta = CUBLAS_OP_T, tb = CUBLAS_OP_N;
-        if (l.desc_set(desc, CUBLASLT_MATMUL_DESC_TRANSA, &ta, sizeof ta) != CUBLAS_STATUS_SUCCESS) break;
-        if (l.desc_set(desc, CUBLASLT_MATMUL_DESC_TRANSB, &tb, sizeof tb) != CUBLAS_STATUS_SUCCESS) break;
-        if (l.layout_create(&la, CUDA_R_16BF, K, N, K) != CUBLAS_STATUS_SUCCESS) break;   // w: K x N, column-major
-        if (l.layout_create(&lb, CUDA_R_16BF, K, T, K) != CUBLAS_STATUS_SUCCESS) break;   // x parts: K x T
-        if (l.layout_create(&lc, CUDA_R_32F, N, T, N) != CUBLAS_STATUS_SUCCESS) break;    // out: N x T
-        if (l.pref_create(&pref) != CUBLAS_STATUS_SUCCESS) break;
-        const size_t ws = LT_WORKSPACE;
-        if (l.pref_set(pref, CUBLASLT_MATMUL_PREF_MAX_WORKSPACE_BYTES, &ws, sizeof ws) != CUBLAS_STATUS_SUCCESS) break;
-        cublasLtMatmulHeuristicResult_t heur{};
-        int found = 0;
-        if (l.heuristic((cublasLtHandle_t)ctx->lt_handle, desc, la, lb, lc, lc, pref, 1, &heur, &found) != CUBLAS_STATUS_SUCCESS || found == 0)
-            break;
-        const float one = 1.0f, zero = 0.0f;
-        cublasStatus_t st = l.matmul((cublasLtHandle_t)ctx->lt_handle, desc, &one, w, la, hi, lb, &zero, out, lc, out, lc, &heur.algo,
-                                     ctx->lt_workspace, LT_WORKSPACE, ctx->stream);
-        if (st == CUBLAS_STATUS_SUCCESS)
-            st = l.matmul((cublasLtHandle_t)ctx->lt_handle, desc, &one, w, la, lo, lb, &one, out, lc, out, lc, &heur.algo,
-                          ctx->lt_workspace, LT_WORKSPACE, ctx->stream);
-        if (st != CUBLAS_STATUS_SUCCESS) {
-            result = fail(ctx, YX_ERR_CUDA, "matmul: cublasLtMatmul failed with status " + std::to_string((int)st));
-            break;
-        }
-        ctx->launches += 2;
-        ctx->last_launch = yx_ctx::LAST_OTHER;
-        result = YX_OK;
-    } while (false);
-    if (pref) l.pref_destroy(pref);
-    if (lc) l.layout_destroy(lc);
-    if (lb) l.layout_destroy(lb);
-    if (la) l.layout_destroy(la);
-    if (desc) l.desc_destroy(desc);
-    return result;
-}
-
 template <int NT>
 int launch_matmul_rows(yx_ctx *ctx, const float *x, const __nv_bfloat16 *w, uint32_t T, uint32_t N, uint32_t K, float *part,
                        uint32_t kc, uint32_t chunks) {
@@ -626,8 +493,8 @@ int matmul_impl(yx_ctx *ctx, const float *x, const void *w_bf16, uint32_t T, uin
     if (K % (MM_STEP * MM_AHEAD) != 0 || ((uintptr_t)w & 15u) != 0 || ((uintptr_t)x & 7u) != 0) {
         float *dst = out;
         if (glu) {
-            if (int rc = ensure_buffer(ctx, (void **)&ctx->mm_part, &ctx->mm_part_cap, (size_t)T * N * sizeof(float))) return rc;
-            dst = ctx->mm_part;
+            if (int rc = ensure_buffer(ctx, (void **)&ctx->mm_sums, &ctx->mm_sums_cap, (size_t)T * N * sizeof(float))) return rc;
+            dst = ctx->mm_sums;
         }
         const uint64_t threads = (uint64_t)T * N * 32;
         matmul_any_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, ctx->stream>>>(x, w, T, N, K, dst);
@@ -639,21 +506,14 @@ int matmul_impl(yx_ctx *ctx, const float *x, const void *w_bf16, uint32_t T, uin
         }
         return YX_OK;
     }
+    // More rows than the row kernel takes at once: that one would stream the weights once for every 32 of them.
     if (T > MM_MAX_T && ctx->tuning.force_path != 2) {
-        float *dst = out;
-        if (glu) {
-            if (int rc = ensure_buffer(ctx, (void **)&ctx->mm_part, &ctx->mm_part_cap, (size_t)T * N * sizeof(float))) return rc;
-            dst = ctx->mm_part;
-        }
-        const int rc = matmul_lt(ctx, x, w, T, N, K, dst);
-        if (rc > 0) return rc;
-        if (rc == YX_OK) {
-            if (!glu) return YX_OK;
-            const uint64_t n = (uint64_t)T * cols;
-            swiglu_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(dst, T, cols, out);
-            return launched(ctx, "swiglu kernel");
-        }
-        // (no cuBLASLt, or no kernel of its for this shape: the row kernel below)
+        if (!glu || cols % 16 == 0) return launch_matmul_tc(ctx, x, w, T, N, K, glu != 0, out);
+        if (int rc = ensure_buffer(ctx, (void **)&ctx->mm_sums, &ctx->mm_sums_cap, (size_t)T * N * sizeof(float))) return rc;
+        if (int rc = launch_matmul_tc(ctx, x, w, T, N, K, false, ctx->mm_sums)) return rc;
+        const uint64_t n = (uint64_t)T * cols;
+        swiglu_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(ctx->mm_sums, T, cols, out);
+        return launched(ctx, "swiglu kernel");
     }
     // K is cut into chunks (an item is 16 weight rows of one chunk) until every resident warp has
     // a few items to take, which evens the warps' loads out; no more than eight chunks, whose
@@ -681,11 +541,6 @@ int matmul_impl(yx_ctx *ctx, const float *x, const void *w_bf16, uint32_t T, uin
 }
 
 }  // namespace
-
-void release_matmul_library(yx_ctx *ctx) {
-    if (ctx->lt_handle && lt().ok()) lt().destroy((cublasLtHandle_t)ctx->lt_handle);
-    ctx->lt_handle = nullptr;
-}
 
 }  // namespace yx
 

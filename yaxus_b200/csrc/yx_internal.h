@@ -337,13 +337,15 @@ struct yx_ctx {
     size_t q_tmp_cap = 0;
     uint32_t *counters = nullptr;   // arrival counters of the fused merge; all zero between launches
     size_t counters_cap = 0;
-    float *mm_part = nullptr;              // per-k-chunk partial sums of the matmul
+    float *mm_part = nullptr;              // partial sums of the matmul kernels
     size_t mm_part_cap = 0;
-    void *mm_packed = nullptr;             // the pass rows of a matmul as bf16 MMA fragments
+    void *mm_packed = nullptr;             // the pass rows of a matmul as two bf16 parts
     size_t mm_packed_cap = 0;
-    void *lt_handle = nullptr;             // cublasLtHandle_t, made at the first matmul of many rows
-    void *lt_workspace = nullptr;
-    size_t lt_workspace_cap = 0;
+    float *mm_sums = nullptr;              // gate and up rows of a GLU whose kernel writes them out unfused
+    size_t mm_sums_cap = 0;
+    uint32_t *mm_counters = nullptr;       // arrivals at the matmul tiles several CTAs share; zero between launches
+    size_t mm_counters_cap = 0;
+    int mm_pairs[2] = {0, 0};              // CTA pairs of the matmul kernel (plain, GLU) that fit the chip together
     uint32_t *idx_dev = nullptr;           // token ids / row indices / argmax parts of the model operators
     size_t idx_cap = 0;
     uint32_t *pick_counters = nullptr;     // argmax: arrivals per row, zero between launches
@@ -369,8 +371,8 @@ int ensure_buffer(yx_ctx *ctx, void **buf, size_t *cap, size_t bytes);
 // yx_attend over the keys [key_lo, key_hi) only: what one rank alone has to do for yx_attend_allgather.
 int attend_key_range(yx_ctx *ctx, yx_kv *kv, int layer, const void *q, int q_dtype, int hq, int64_t window, uint64_t key_lo,
                      uint64_t key_hi, void *out, int out_dtype);
-// Destroys the context's cuBLASLt handle, if it made one.
-void release_matmul_library(yx_ctx *ctx);
+// out = x . w^T on the tensor cores for many rows (matmul_tc.cu says what it takes).
+int launch_matmul_tc(yx_ctx *ctx, const float *x, const void *w, uint32_t T, uint32_t N, uint32_t K, bool glu, float *out);
 
 // Kernel launchers (each returns a yx_error and counts its launches in ctx->launches).
 int launch_append(yx_ctx *ctx, yx_kv *kv, int layer, const void *k_rows, const void *v_rows, int src_dtype);

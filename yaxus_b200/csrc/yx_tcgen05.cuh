@@ -64,20 +64,16 @@ __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// Tiled TMA copies of a three-dimensional box, and the same box asked into L2 only.
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const void *map, int x, int y, int z, uint32_t bar) {
-    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
-                 "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar)
-                 : "memory");
-}
-// (of one CTA of a pair, signalling a barrier that may be its partner's)
+// Tiled TMA copies by one CTA of a pair, signalling a barrier that may be its partner's.
 __device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const void *map, int x, int y, int z, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
                  "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar)
                  : "memory");
 }
-__device__ __forceinline__ void tma_prefetch_3d(const void *map, int x, int y, int z) {
-    asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(map), "r"(x), "r"(y), "r"(z) : "memory");
+__device__ __forceinline__ void tma_load_4d_pair(uint32_t dst, const void *map, int x, int y, int z, int w, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst),
+                 "l"(map), "r"(x), "r"(y), "r"(z), "r"(w), "r"(bar)
+                 : "memory");
 }
 __device__ __forceinline__ void prefetch_tensormap(const void *map) { asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory"); }
 
