@@ -1,5 +1,5 @@
-"""The many-row matmul at the edges of its tiles: ragged weight rows and pass rows, one and two tiles of
-pass rows, tiles shared along k by several CTA pairs, whole rounds before and after them."""
+"""The matmul kernels at the edges of their tiles: ragged weight rows and pass rows, one and two tiles of
+pass rows, tiles shared along k by several CTAs or CTA pairs, whole tiles before and after them."""
 import numpy as np
 import pytest
 import torch
@@ -27,6 +27,9 @@ def inputs(oracle, t, n, k):
 
 
 @pytest.mark.parametrize("t,n,k", [
+    # few rows: each size of operand; one k step a CTA, a tile of 148 shares and more, several whole tiles a CTA
+    (1, 1, 128), (7, 127, 256), (8, 129, 1024), (9, 300, 128), (16, 1000, 640), (17, 4100, 256), (32, 257, 1152),
+    (1, 128, 19200), (3, 40000, 128), (32, 39000, 128),
     (33, 1, 128), (64, 255, 128), (65, 257, 384), (256, 256, 1024), (257, 300, 640),   # fewer tiles than pairs
     (40, 19300, 128), (300, 9700, 256),                                                # rounds and a remainder
     (513, 6400, 128), (34, 18944, 128)])                                               # (the last: whole rounds where 74 pairs fit)
@@ -40,7 +43,7 @@ def test_matmul_tiles(backend, oracle, t, n, k):
     assert np.array_equal(backend.to_host(backend.matmul(xd, w)), first)
 
 
-@pytest.mark.parametrize("t,inner,k", [(33, 16, 128), (48, 144, 1024), (257, 1040, 256), (100, 24, 256), (35, 9696, 128)])
+@pytest.mark.parametrize("t,inner,k", [(1, 16, 128), (8, 1040, 256), (13, 48, 1024), (32, 9696, 128), (5, 24, 256), (33, 16, 128), (48, 144, 1024), (257, 1040, 256), (100, 24, 256), (35, 9696, 128)])
 def test_glu_tiles(backend, oracle, t, inner, k):
     x, w_bits = inputs(oracle, t, 2 * inner, k)
     w = backend.load_weight(w_bits)
@@ -55,11 +58,12 @@ def test_glu_tiles(backend, oracle, t, inner, k):
     assert np.array_equal(backend.to_host(backend.matmul_glu(xd, w)), got)
 
 
-def test_unaligned_rows(backend, oracle):
+@pytest.mark.parametrize("t", [5, 70])
+def test_unaligned_rows(backend, oracle, t):
     # pass rows that start 8 bytes past a 16-byte boundary
-    x, w_bits = inputs(oracle, 70, 200, 256)
-    store = torch.zeros(70 * 256 + 2, dtype=torch.float32, device=backend.device)
-    xd = store[2:].view(70, 256)
+    x, w_bits = inputs(oracle, t, 200, 256)
+    store = torch.zeros(t * 256 + 2, dtype=torch.float32, device=backend.device)
+    xd = store[2:].view(t, 256)
     xd.copy_(torch.from_numpy(x))
     got = backend.to_host(backend.matmul(xd, backend.load_weight(w_bits)))
     assert (np.abs(got - oracle.matmul(x, w_bits)) <= TOL * magnitudes(x, w_bits)).all()

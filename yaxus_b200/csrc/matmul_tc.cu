@@ -370,6 +370,280 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float *__restrict
     lo[idx] = make_uint4(l[0], l[1], l[2], l[3]);
 }
 
+// ---- passes of few rows ------------------------------------------------------------------------------------
+//
+// At most 32 pass rows: the weights stream through the chip once and everything else must stay out of their way.
+// One launch: the activations are split into their bf16 parts on the way into shared memory by eight warps, each
+// with every eighth k step, so that eight steps' loads are in flight; a step's operand is the high parts' rows and
+// the low parts' rows one below the other, one MMA per 16 k takes both, and the epilogue adds the two halves of
+// the accumulator.  128 weight rows by 64 k make a stage; the k steps of all tiles are laid end to end and cut
+// into one equal share a CTA, so that every SM streams the same number of bytes whatever N and K are.
+// A share that ends inside a tile leaves its sums in scratch, and the CTA that comes last at a tile adds them up
+// in the order of k.
+// The kernel starts under the one ahead of it and asks its first stages into L2 before it waits: weights are not
+// written by the kernel ahead, and even if they were, L2 is where such writes land.
+//
+// Bound by HBM from some 200 MB on (one row on 28672 x 4096: 45 us, the part above a launch's fixed 8 to 12 us at
+// 7.2 TB/s), by a chain of latencies below.  The kernel with weights straight from global memory into mma.sync
+// fragments, a packing kernel before it and a finishing kernel behind took 58 us for sixteen rows of that weight;
+// steps went from 419 to 374 us (one row, large), 538 to 440 us (sixteen rows), 417 to 340 us (one row, small).
+constexpr int ROWS_THREADS = 14 * 32;
+constexpr int ROWS_CONVERT_WARP = 6, ROWS_CONVERTERS = 8;
+constexpr uint32_t ROWS_M = 128;
+
+struct RowsArgs {
+    const float *x;
+    uint32_t T, K, cols, ksteps, units, ctas, stages;
+    uint32_t x_vec16;
+    float *out;
+    float *part;          // [2 * ctas shares][TP][128]
+    uint32_t *counters;   // one a tile, zero between launches
+    yx_dev_status *status;
+};
+__device__ __forceinline__ uint32_t share_begin(const RowsArgs &a, uint32_t p) { return (uint32_t)((uint64_t)p * a.units / a.ctas); }
+__device__ __forceinline__ uint32_t share_owner(const RowsArgs &a, uint32_t u) { return (uint32_t)((((uint64_t)u + 1) * a.ctas - 1) / a.units); }
+
+// TP pass rows of this lane's weight row.
+template <int TP, bool GLU>
+__device__ __forceinline__ void store_few(const RowsArgs &a, const float (&v)[TP], uint32_t row, int lane) {
+    if constexpr (!GLU) {
+        if (row >= a.cols) return;
+#pragma unroll
+        for (int i = 0; i < TP; i++)
+            if (i < (int)a.T) a.out[(size_t)i * a.cols + row] = v[i];
+    } else {
+        // (see store_rows: the lower half of the warp finishes the first half of the pass rows)
+        const uint32_t col = (row >> 5) * GLU_GROUP + (lane & 15), t = lane < 16 ? 0 : TP / 2;
+#pragma unroll
+        for (int i = 0; i < TP / 2; i++) {
+            const float other = __shfl_xor_sync(0xffffffffu, lane < 16 ? v[TP / 2 + i] : v[i], 16);
+            const float g = lane < 16 ? v[i] : other, u = lane < 16 ? other : v[TP / 2 + i];
+            if (col < a.cols && t + i < a.T) a.out[(size_t)(t + i) * a.cols + col] = g / (1.0f + expf(-g)) * u;
+        }
+    }
+}
+
+template <int TP, bool GLU>
+__global__ void __launch_bounds__(ROWS_THREADS, 1)
+matmul_rows_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ RowsArgs a) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    __shared__ __align__(8) uint64_t bar_store[2 * TC_MAX_STAGES + 4];
+    __shared__ uint32_t tmem_base_s;
+    __shared__ int abort_flag;
+    __shared__ int last_s;
+    constexpr uint32_t NB = 2 * TP, X_BYTES = NB * 128, STAGE = W_BYTES + X_BYTES;
+    constexpr uint32_t TMEM = 2 * NB < 32 ? 32 : 2 * NB;   // two accumulators
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t S = a.stages, base = smem_u32(smem);
+    const uint32_t b_full = smem_u32(bar_store), b_empty = b_full + 8 * TC_MAX_STAGES;
+    const uint32_t b_acc_full = b_empty + 8 * TC_MAX_STAGES, b_acc_empty = b_acc_full + 16;
+    volatile int *abortp = &abort_flag;
+    const uint32_t u0 = share_begin(a, blockIdx.x), u1 = share_begin(a, blockIdx.x + 1);
+
+    auto weight_rows = [&](uint32_t u, int &x, int &y, int &z) {
+        const uint32_t tile = u / a.ksteps;
+        x = (int)((u - tile * a.ksteps) * TC_KSTEP);
+        y = GLU ? 0 : (int)(tile * ROWS_M);
+        z = GLU ? (int)(tile * (ROWS_M / (2 * GLU_GROUP))) : 0;
+    };
+    if (warp == 4 && lane == 0) {
+        prefetch_tensormap(&w_map);
+        for (uint32_t u = u0; u < u1 && u - u0 < S; u++) {
+            int x, y, z;
+            weight_rows(u, x, y, z);
+            tma_prefetch_4d(&w_map, x, y, 0, z);
+        }
+    }
+    if (threadIdx.x == 0) {
+        abort_flag = 0;
+        for (uint32_t s = 0; s < S; s++) {
+            mbar_init(b_full + 8 * s, 2);    // the weights' copy and the converting warp
+            mbar_init(b_empty + 8 * s, 1);
+        }
+        for (int b = 0; b < 2; b++) {
+            mbar_init(b_acc_full + 8 * b, 1);
+            mbar_init(b_acc_empty + 8 * b, 4);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 5) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)), "n"(TMEM) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_base_s;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+
+    if (warp == 4) {
+        // ---- weights --------------------------------------------------------------------------
+        if (lane == 0) {
+            uint32_t s = 0, phase = 0;
+            for (uint32_t u = u0; u < u1; u++) {
+                if (u - u0 >= S) mbar_wait(b_empty + 8 * s, phase ^ 1u, abortp, a.status, 511);
+                if (*abortp) break;
+                int x, y, z;
+                weight_rows(u, x, y, z);
+                mbar_expect_tx(b_full + 8 * s, W_BYTES);
+                tma_load_4d(base + s * STAGE, &w_map, x, y, 0, z, b_full + 8 * s);
+                if (++s == S) {
+                    s = 0;
+                    phase ^= 1u;
+                }
+            }
+        }
+    } else if (warp == 5) {
+        // ---- MMA issuer -----------------------------------------------------------------------
+        if (lane == 0) {
+            constexpr uint32_t idesc = f16_instr_desc(true, false, ROWS_M, NB);
+            uint32_t s = 0, phase = 0, n = 0;
+            for (uint32_t u = u0; u < u1 && !*abortp; n++) {
+                const uint32_t end = min(u1, (u / a.ksteps + 1) * a.ksteps);
+                const uint32_t buf = n & 1u, acc = tmem + buf * NB;
+                if (n >= 2) mbar_wait(b_acc_empty + 8 * buf, ((n >> 1) - 1) & 1u, abortp, a.status, 512);
+                tc_fence_after();
+                for (uint32_t first = u; u < end; u++) {
+                    mbar_wait(b_full + 8 * s, phase, abortp, a.status, 513);
+                    if (*abortp) break;
+                    tc_fence_after();
+                    const uint32_t w_lo = desc_lo(base + s * STAGE, 0), x_lo = w_lo + W_BYTES / 16;
+#pragma unroll
+                    for (uint32_t kk = 0; kk < 4; kk++) umma_ss_lo(acc, w_lo + 2 * kk, x_lo + 2 * kk, idesc, u > first || kk > 0);
+                    umma_commit(b_empty + 8 * s);
+                    if (++s == S) {
+                        s = 0;
+                        phase ^= 1u;
+                    }
+                }
+                umma_commit(b_acc_full + 8 * buf);
+            }
+        }
+    } else if (warp >= ROWS_CONVERT_WARP) {
+        // ---- activations: every eighth step is this warp's ------------------------------------------
+        for (uint32_t u = u0 + (uint32_t)(warp - ROWS_CONVERT_WARP); u < u1; u += ROWS_CONVERTERS) {
+            const uint32_t it = u - u0, s = it % S, use = it / S;
+            const float *src = a.x + (size_t)(u % a.ksteps) * TC_KSTEP;
+            constexpr int R = TP / 4;          // 16-byte operand chunks (eight k of a pass row) a lane
+            float v[R][8];
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const uint32_t t = r * 4 + (lane >> 3);
+                if (t >= a.T) continue;        // (rows past T only reach accumulator columns that nobody reads)
+                const float *p = src + (size_t)t * a.K + (lane & 7) * 8;
+                if (a.x_vec16) {
+                    *(float4 *)&v[r][0] = *(const float4 *)p;
+                    *(float4 *)&v[r][4] = *(const float4 *)(p + 4);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 4; j++) *(float2 *)&v[r][2 * j] = *(const float2 *)(p + 2 * j);
+                }
+            }
+            if (use > 0) mbar_wait(b_empty + 8 * s, (use - 1) & 1u, abortp, a.status, 514);
+            if (__any_sync(0xffffffffu, *abortp)) break;
+            unsigned char *dst = smem + s * STAGE + W_BYTES;
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const uint32_t t = r * 4 + (lane >> 3);
+                if (t >= a.T) continue;
+                uint32_t h[4], l[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    h[j] = pack2<true>(v[r][2 * j], v[r][2 * j + 1]);
+                    const float2 b = unpack2<true>(h[j]);
+                    l[j] = pack2<true>(v[r][2 * j] - b.x, v[r][2 * j + 1] - b.y);
+                }
+                unsigned char *at = dst + t * 128 + (((lane & 7) ^ (t & 7)) << 4);
+                *(uint4 *)at = make_uint4(h[0], h[1], h[2], h[3]);
+                *(uint4 *)(at + TP * 128) = make_uint4(l[0], l[1], l[2], l[3]);
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(b_full + 8 * s);
+        }
+    } else {
+        // ---- epilogue -------------------------------------------------------------------------
+        uint32_t n = 0;
+        for (uint32_t u = u0; u < u1; n++) {
+            const uint32_t tile = u / a.ksteps, end = min(u1, (tile + 1) * a.ksteps);
+            const bool whole = end - u == a.ksteps;
+            const uint32_t buf = n & 1u, acc = tmem + buf * NB + ((uint32_t)warp << 21), wr = warp * 32 + lane, row = tile * ROWS_M + wr;
+            u = end;
+            mbar_wait(b_acc_full + 8 * buf, (n >> 1) & 1u, abortp, a.status, 515);
+            __syncwarp();   // (a wait that ran out does not stop these warps: their barriers below count all of them)
+            tc_fence_after();
+            float v[TP];
+            if constexpr (TP == 8) {
+                uint32_t r[16];
+                tmem_ld16(acc, r);
+                tmem_ld_wait();
+#pragma unroll
+                for (int i = 0; i < 8; i++) v[i] = __uint_as_float(r[i]) + __uint_as_float(r[8 + i]);
+            } else {
+#pragma unroll
+                for (int h = 0; h < TP / 16; h++) {
+                    uint32_t r[16], q[16];
+                    tmem_ld16(acc + 16 * h, r);
+                    tmem_ld16(acc + TP + 16 * h, q);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int i = 0; i < 16; i++) v[16 * h + i] = __uint_as_float(r[i]) + __uint_as_float(q[i]);
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(b_acc_empty + 8 * buf);
+            if (whole) {
+                store_few<TP, GLU>(a, v, row, lane);
+                continue;
+            }
+            auto share = [&](uint32_t q) {   // share of CTA q in this tile: its first piece or its last
+                return a.part + (size_t)(2 * q + (tile != share_begin(a, q) / a.ksteps)) * TP * 128u + wr;
+            };
+            float *mine = share(blockIdx.x);
+#pragma unroll
+            for (int i = 0; i < TP; i++)
+                if (i < (int)a.T) __stcg(mine + i * 128, v[i]);
+            const uint32_t q0 = share_owner(a, tile * a.ksteps), q1 = share_owner(a, (tile + 1) * a.ksteps - 1);
+            __threadfence();
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+            if (threadIdx.x == 0) {
+                const int last = atomicAdd(a.counters + tile, 1u) == q1 - q0;
+                if (last) a.counters[tile] = 0u;
+                last_s = last;
+            }
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+            const bool last = last_s != 0;
+            if (!last) continue;
+            __threadfence();
+#pragma unroll
+            for (int i = 0; i < TP; i++) v[i] = 0.0f;
+            constexpr int B = 64 / TP;   // shares read at once
+            for (uint32_t q = q0; q <= q1; q += B) {
+                float w[B][TP];
+#pragma unroll
+                for (int b = 0; b < B; b++) {
+                    const float *src = share(min(q + b, q1));
+#pragma unroll
+                    for (int i = 0; i < TP; i++) w[b][i] = i < (int)a.T && q + b <= q1 ? __ldcg(src + i * 128) : 0.0f;
+                }
+#pragma unroll
+                for (int b = 0; b < B; b++)
+#pragma unroll
+                    for (int i = 0; i < TP; i++) v[i] += w[b][i];
+            }
+            store_few<TP, GLU>(a, v, row, lane);
+        }
+    }
+    __syncwarp();
+    if (*abortp)
+        for (int i = 0; i < 64; i++) __nanosleep(1000);   // copies and products in flight come to rest
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 5) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(TMEM) : "memory");
+}
+
 using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
                                  const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -492,11 +766,53 @@ int matmul_pair_rows(yx_ctx *ctx, const float *x, const void *w, uint32_t T, uin
     return launch_dependent(ctx, "matmul kernel launch", matmul_pair_kernel<GLU>, dim3(grid), dim3(TC_THREADS), a.stages * stage_bytes, w_map, x_map, a);
 }
 
+template <int TP, bool GLU>
+int matmul_few_rows(yx_ctx *ctx, const float *x, const void *w, uint32_t T, uint32_t N, uint32_t K, float *out) {
+    constexpr uint32_t stage_bytes = W_BYTES + 2 * TP * 128, stages = std::min<uint32_t>(TC_MAX_STAGES, TC_SMEM_BUDGET / stage_bytes);
+    auto *kernel = matmul_rows_kernel<TP, GLU>;
+    bool &configured = ctx->mm_rows_configured[GLU][TP / 16];
+    if (!configured) {
+        if (int rc = check_cuda(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, stages * stage_bytes),
+                                "matmul: shared memory attribute"))
+            return rc;
+        configured = true;
+    }
+    RowsArgs a{};
+    a.x = x;
+    a.T = T;
+    a.K = K;
+    a.cols = GLU ? N / 2 : N;
+    a.ksteps = K / TC_KSTEP;
+    const uint32_t tiles = (N + ROWS_M - 1) / ROWS_M;
+    a.units = tiles * a.ksteps;
+    a.ctas = std::min((uint32_t)ctx->sm_count, std::max(1u, a.units / 2));
+    a.stages = stages;
+    a.x_vec16 = ((uintptr_t)x & 15u) == 0;
+    a.out = out;
+    a.status = ctx->dev_status;
+    if (int rc = ensure_buffer(ctx, (void **)&ctx->mm_part, &ctx->mm_part_cap, (size_t)2 * a.ctas * TP * 128 * sizeof(float))) return rc;
+    if (int rc = ensure_counters(ctx, tiles)) return rc;
+    a.part = ctx->mm_part;
+    a.counters = ctx->mm_counters;
+    CUtensorMap w_map;
+    if (int rc = encode_weights(ctx, &w_map, w, N, K, GLU)) return rc;
+    ctx->last_launch = yx_ctx::LAST_OTHER;
+    return launch_dependent(ctx, "matmul kernel launch", kernel, dim3(a.ctas), dim3(ROWS_THREADS), stages * stage_bytes, w_map, a);
+}
+
+template <bool GLU>
+int matmul_tc(yx_ctx *ctx, const float *x, const void *w, uint32_t T, uint32_t N, uint32_t K, float *out) {
+    if (T <= 8) return matmul_few_rows<8, GLU>(ctx, x, w, T, N, K, out);
+    if (T <= 16) return matmul_few_rows<16, GLU>(ctx, x, w, T, N, K, out);
+    if (T <= 32) return matmul_few_rows<32, GLU>(ctx, x, w, T, N, K, out);
+    return matmul_pair_rows<GLU>(ctx, x, w, T, N, K, out);
+}
+
 }  // namespace
 
 // Takes K a multiple of 64, w 16-byte aligned, x 8-byte aligned; with `glu`, a multiple of 16 result columns.
 int launch_matmul_tc(yx_ctx *ctx, const float *x, const void *w, uint32_t T, uint32_t N, uint32_t K, bool glu, float *out) {
-    return glu ? matmul_pair_rows<true>(ctx, x, w, T, N, K, out) : matmul_pair_rows<false>(ctx, x, w, T, N, K, out);
+    return glu ? matmul_tc<true>(ctx, x, w, T, N, K, out) : matmul_tc<false>(ctx, x, w, T, N, K, out);
 }
 
 }  // namespace yx

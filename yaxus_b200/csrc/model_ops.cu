@@ -3,18 +3,8 @@
 // (crates/yaxus-backend-cpu/src/lib.rs:485-562): embedding gather, RMSNorm, the fused residual
 // step, matmul against bf16 weights, SwiGLU, add, row gather, argmax.
 //
-// All of them are bandwidth-bound.  The only one with real traffic is the matmul: at decode a
-// pass has at most 16 rows, so `x [T,K] . w[N,K]^T` streams the weight matrix once and does
-// 2 T flops per weight byte.  It is taken transposed, out^T = W x^T, with `mma.sync.m16n8k16`:
-// the 16-row side holds weight rows (always full), the 8-column side holds pass rows, as in the
-// split-key attention kernel.  Activations stay f32 in the interface; a small kernel first turns
-// them into a high and a low bf16 part (x = hi + lo to 16 bits of mantissa), laid out in the
-// order the MMA's B fragments want, and every weight fragment is used twice.
-// Weights go from global memory straight into A fragments with 16-byte loads: a thread takes
-// eight consecutive k of one weight row, which permutes k inside a step the same way for both
-// operands, so the products pair up correctly.
-//
-// Passes of more than 32 rows (prompt chunks, verification) go to the tcgen05 kernel of matmul_tc.cu.
+// All of them are bandwidth-bound or a chain of latencies.  The one with real traffic, the matmul, is in
+// matmul_tc.cu; here is its form for shapes that one does not take.
 #include <cuda_bf16.h>
 #include <string.h>
 
@@ -26,153 +16,6 @@ namespace yx {
 namespace {
 
 using namespace dev;
-
-constexpr int MM_WARPS = 4;
-constexpr int MM_AHEAD = 4;               // steps of weights in flight per thread
-constexpr int MM_CTAS_PER_SM = 5;
-constexpr int MM_STEP = 32;              // k per warp step: one 16-byte load per thread and row half
-constexpr int MM_PAIR = 64;              // two steps: the four threads of a weight row read one whole 128-byte line
-constexpr int MM_MAX_T = 32;             // pass rows per launch (four 8-column tiles)
-
-__device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                         uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-__device__ __forceinline__ uint4 ldg_stream(const void *p) {
-    uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-    return v;
-}
-
-// The activations of up to 32 pass rows as the MMA's B fragments want them: per 32-k step and
-// 8-row column tile a 512-byte block of high parts and one of low parts, lane-major (lane =
-// 4 g + t holds the eight k that thread t of a weight row's four loads in that step: steps come in
-// pairs over 64 k, thread t owning k = 16 t .. 16 t + 15 of the pair, the lower eight in the even step).
-// Rows past T are zero.
-template <int NT>
-__global__ void pack_rows_kernel(const float *__restrict__ x, uint32_t T, uint32_t K, uint4 *__restrict__ packed) {
-    const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x;   // one thread per 16-byte pair of blocks
-    const uint32_t steps = K / MM_STEP;
-    if (idx >= steps * NT * 32u) return;
-    const uint32_t lane = idx & 31u, tile = (idx >> 5) % NT, s = (idx >> 5) / NT;
-    const uint32_t n = tile * 8 + (lane >> 2), k0 = (s >> 1) * MM_PAIR + (lane & 3u) * 16 + (s & 1u) * 8;
-    uint32_t hi[4], lo[4];
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-        float v[2] = {0.0f, 0.0f};
-        if (n < T) {
-            const float2 p = *(const float2 *)(x + (size_t)n * K + k0 + 2 * j);
-            v[0] = p.x;
-            v[1] = p.y;
-        }
-        const __nv_bfloat16 h0 = __float2bfloat16_rn(v[0]), h1 = __float2bfloat16_rn(v[1]);
-        const __nv_bfloat16 l0 = __float2bfloat16_rn(v[0] - __bfloat162float(h0)), l1 = __float2bfloat16_rn(v[1] - __bfloat162float(h1));
-        hi[j] = (uint32_t)__bfloat16_as_ushort(h0) | ((uint32_t)__bfloat16_as_ushort(h1) << 16);
-        lo[j] = (uint32_t)__bfloat16_as_ushort(l0) | ((uint32_t)__bfloat16_as_ushort(l1) << 16);
-    }
-    uint4 *dst = packed + ((size_t)(s * NT + tile) * 2u) * 32u + lane;
-    dst[0] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-    dst[32] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-}
-
-// part[ky][t][n] = sum over k-chunk ky of x[t][k] * w[n][k].  NT = 8-column tiles of pass rows.
-// The work is cut into items of 16 weight rows x one chunk of kc columns, dealt round-robin to the
-// warps of a grid that just fills the machine.  A warp's weights come straight from global memory
-// into A fragments, AHEAD steps in flight, and the prefetch runs on into the warp's next item, so
-// the stream never drains; the packed activations are read through L1.  kc is a multiple of 32 AHEAD.
-template <int NT>
-__global__ void __launch_bounds__(MM_WARPS * 32, 5) matmul_rows_kernel(const uint4 *__restrict__ packed, const __nv_bfloat16 *__restrict__ w,
-                                                                        uint32_t T, uint32_t N, uint32_t K, uint32_t kc, uint32_t chunks,
-                                                                        float *__restrict__ part) {
-    constexpr int AHEAD = MM_AHEAD;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
-    const uint32_t steps = kc / MM_STEP;
-    const uint32_t total = ((N + 15u) / 16u) * chunks, n_warps = gridDim.x * MM_WARPS;
-    uint32_t item = blockIdx.x * MM_WARPS + warp;
-    if (item >= total) return;
-    auto at = [](uint32_t s) { return (size_t)(s >> 1) * MM_PAIR + (s & 1u) * 8; };   // element offset of step s
-    // Rows past N repeat the last row (their results are not stored).
-    auto row_ptr = [&](uint32_t it, uint32_t half) {
-        const uint32_t r = min((it / chunks) * 16u + g + half * 8u, N - 1u);
-        return w + (size_t)r * K + (size_t)(it % chunks) * kc + t4 * 16;
-    };
-    // The prefetch position: AHEAD steps ahead of the consumer.
-    uint32_t pf_item = item, pf_step = 0;
-    const __nv_bfloat16 *pf_a = row_ptr(item, 0), *pf_b = row_ptr(item, 1);
-    uint4 wa[AHEAD], wb[AHEAD];
-#pragma unroll
-    for (int i = 0; i < AHEAD; i++) {   // (steps >= AHEAD)
-        wa[i] = ldg_stream(pf_a + at(pf_step));
-        wb[i] = ldg_stream(pf_b + at(pf_step));
-        pf_step++;
-    }
-    for (; item < total; item += n_warps) {
-        const uint32_t ky = item % chunks, row0 = (item / chunks) * 16u;
-        const uint4 *xp = packed + (size_t)ky * steps * NT * 64u + lane;
-        float acc[NT][4];
-#pragma unroll
-        for (int n = 0; n < NT; n++) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.0f;
-        for (uint32_t s0 = 0; s0 < steps; s0 += AHEAD) {
-#pragma unroll
-            for (int i = 0; i < AHEAD; i++) {
-                const uint32_t s = s0 + i;
-                const uint4 a = wa[i], b = wb[i];
-                if (pf_step == steps) {   // on to this warp's next item
-                    pf_step = 0;
-                    pf_item += n_warps;
-                    if (pf_item < total) {
-                        pf_a = row_ptr(pf_item, 0);
-                        pf_b = row_ptr(pf_item, 1);
-                    }
-                }
-                if (pf_item < total) {
-                    wa[i] = ldg_stream(pf_a + at(pf_step));
-                    wb[i] = ldg_stream(pf_b + at(pf_step));
-                    pf_step++;
-                }
-#pragma unroll
-                for (int n = 0; n < NT; n++) {
-                    const uint4 hi = __ldg(xp + ((size_t)s * NT + n) * 64u);
-                    const uint4 lo = __ldg(xp + ((size_t)s * NT + n) * 64u + 32u);
-                    mma_bf16(acc[n], a.x, b.x, a.y, b.y, hi.x, hi.y);
-                    mma_bf16(acc[n], a.z, b.z, a.w, b.w, hi.z, hi.w);
-                    mma_bf16(acc[n], a.x, b.x, a.y, b.y, lo.x, lo.y);
-                    mma_bf16(acc[n], a.z, b.z, a.w, b.w, lo.z, lo.w);
-                }
-            }
-        }
-        // c0,c1: weight row g, pass rows 2 t4, 2 t4 + 1 of the tile; c2,c3: weight row g + 8.
-        float *dst = part + (size_t)ky * T * N;
-#pragma unroll
-        for (int n = 0; n < NT; n++) {
-#pragma unroll
-            for (int c = 0; c < 4; c++) {
-                const uint32_t tok = n * 8 + t4 * 2 + (c & 1), row = row0 + g + (c >> 1) * 8;
-                if (tok < T && row < N) dst[(size_t)tok * N + row] = acc[n][c];
-            }
-        }
-    }
-}
-
-// out[t][j] = sum over chunks of part[.][t][j], or with glu: silu(sum[t][j]) * sum[t][I + j], I = N / 2
-// (cpu lib.rs:532-542).
-__global__ void matmul_finish_kernel(const float *__restrict__ part, uint32_t chunks, uint32_t T, uint32_t N, int glu,
-                                     float *__restrict__ out) {
-    const uint32_t cols = glu ? N / 2 : N;
-    const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= T * cols) return;
-    const uint32_t t = idx / cols, j = idx - t * cols;
-    float a = 0.0f, b = 0.0f;
-    for (uint32_t c = 0; c < chunks; c++) {
-        const float *p = part + ((size_t)c * T + t) * N;
-        a += p[j];
-        if (glu) b += p[cols + j];
-    }
-    out[idx] = glu ? a / (1.0f + expf(-a)) * b : a;
-}
 
 // Any shape the tensor-core kernel does not take (K not a multiple of 128): a warp per output.
 __global__ void matmul_any_kernel(const float *__restrict__ x, const __nv_bfloat16 *__restrict__ w, uint32_t T, uint32_t N,
@@ -451,20 +294,6 @@ int launched(yx_ctx *ctx, const char *what) {
     return check_cuda(ctx, cudaGetLastError(), what);
 }
 
-template <int NT>
-int launch_matmul_rows(yx_ctx *ctx, const float *x, const __nv_bfloat16 *w, uint32_t T, uint32_t N, uint32_t K, float *part,
-                       uint32_t kc, uint32_t chunks) {
-    const size_t packed_bytes = (size_t)(K / MM_STEP) * NT * 2 * 512;
-    if (int rc = ensure_buffer(ctx, (void **)&ctx->mm_packed, &ctx->mm_packed_cap, packed_bytes)) return rc;
-    const uint32_t pack_threads = (K / MM_STEP) * NT * 32u;
-    pack_rows_kernel<NT><<<(pack_threads + 255) / 256, 256, 0, ctx->stream>>>(x, T, K, (uint4 *)ctx->mm_packed);
-    if (int rc = launched(ctx, "matmul: activation packing kernel")) return rc;
-    const uint32_t items = ((N + 15u) / 16u) * chunks;
-    const uint32_t grid = std::min<uint32_t>((items + MM_WARPS - 1) / MM_WARPS, (uint32_t)ctx->sm_count * MM_CTAS_PER_SM);
-    matmul_rows_kernel<NT><<<grid, MM_WARPS * 32, 0, ctx->stream>>>((const uint4 *)ctx->mm_packed, w, T, N, K, kc, chunks, part);
-    return launched(ctx, "matmul kernel");
-}
-
 struct Guard {
     int prev = -1;
     explicit Guard(int dev) {
@@ -490,54 +319,24 @@ int matmul_impl(yx_ctx *ctx, const float *x, const void *w_bf16, uint32_t T, uin
     Guard guard(ctx->device);
     const __nv_bfloat16 *w = (const __nv_bfloat16 *)w_bf16;
     const uint32_t cols = glu ? N / 2 : N;
-    if (K % (MM_STEP * MM_AHEAD) != 0 || ((uintptr_t)w & 15u) != 0 || ((uintptr_t)x & 7u) != 0) {
-        float *dst = out;
-        if (glu) {
-            if (int rc = ensure_buffer(ctx, (void **)&ctx->mm_sums, &ctx->mm_sums_cap, (size_t)T * N * sizeof(float))) return rc;
-            dst = ctx->mm_sums;
-        }
+    const bool tensor = K % 128 == 0 && ((uintptr_t)w & 15u) == 0 && ((uintptr_t)x & 7u) == 0;
+    if (tensor && (!glu || cols % 16 == 0)) return launch_matmul_tc(ctx, x, w, T, N, K, glu != 0, out);
+    float *dst = out;
+    if (glu) {
+        if (int rc = ensure_buffer(ctx, (void **)&ctx->mm_sums, &ctx->mm_sums_cap, (size_t)T * N * sizeof(float))) return rc;
+        dst = ctx->mm_sums;
+    }
+    if (tensor) {
+        if (int rc = launch_matmul_tc(ctx, x, w, T, N, K, false, dst)) return rc;
+    } else {
         const uint64_t threads = (uint64_t)T * N * 32;
         matmul_any_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, ctx->stream>>>(x, w, T, N, K, dst);
         if (int rc = launched(ctx, "matmul kernel (any shape)")) return rc;
-        if (glu) {
-            const uint64_t n = (uint64_t)T * cols;
-            swiglu_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(dst, T, cols, out);
-            return launched(ctx, "swiglu kernel");
-        }
-        return YX_OK;
     }
-    // More rows than the row kernel takes at once: that one would stream the weights once for every 32 of them.
-    if (T > MM_MAX_T && ctx->tuning.force_path != 2) {
-        if (!glu || cols % 16 == 0) return launch_matmul_tc(ctx, x, w, T, N, K, glu != 0, out);
-        if (int rc = ensure_buffer(ctx, (void **)&ctx->mm_sums, &ctx->mm_sums_cap, (size_t)T * N * sizeof(float))) return rc;
-        if (int rc = launch_matmul_tc(ctx, x, w, T, N, K, false, ctx->mm_sums)) return rc;
-        const uint64_t n = (uint64_t)T * cols;
-        swiglu_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(ctx->mm_sums, T, cols, out);
-        return launched(ctx, "swiglu kernel");
-    }
-    // K is cut into chunks (an item is 16 weight rows of one chunk) until every resident warp has
-    // a few items to take, which evens the warps' loads out; no more than eight chunks, whose
-    // partial sums the finishing kernel adds up.
-    const uint32_t row_items = (N + 15) / 16, warps = (uint32_t)ctx->sm_count * MM_CTAS_PER_SM * MM_WARPS;
-    uint32_t kc = K;
-    while (kc % (2 * MM_STEP * MM_AHEAD) == 0 && K / (kc / 2) <= 8 && row_items * (K / kc) < 4 * warps) kc /= 2;
-    const uint32_t chunks = K / kc;
-    // Pass rows go 32 at a time; each block of them streams the weights again.
-    for (uint32_t t0 = 0; t0 < T; t0 += MM_MAX_T) {
-        const uint32_t tn = std::min<uint32_t>(MM_MAX_T, T - t0);
-        if (int rc = ensure_buffer(ctx, (void **)&ctx->mm_part, &ctx->mm_part_cap, (size_t)chunks * MM_MAX_T * N * sizeof(float)))
-            return rc;
-        const float *xt = x + (size_t)t0 * K;
-        int rc = tn <= 8    ? launch_matmul_rows<1>(ctx, xt, w, tn, N, K, ctx->mm_part, kc, chunks)
-                 : tn <= 16 ? launch_matmul_rows<2>(ctx, xt, w, tn, N, K, ctx->mm_part, kc, chunks)
-                            : launch_matmul_rows<4>(ctx, xt, w, tn, N, K, ctx->mm_part, kc, chunks);
-        if (rc) return rc;
-        const uint64_t n = (uint64_t)tn * cols;
-        matmul_finish_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(ctx->mm_part, chunks, tn, N, glu,
-                                                                                  out + (size_t)t0 * cols);
-        if (int rc2 = launched(ctx, "matmul finish kernel")) return rc2;
-    }
-    return YX_OK;
+    if (!glu) return YX_OK;
+    const uint64_t n = (uint64_t)T * cols;
+    swiglu_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(dst, T, cols, out);
+    return launched(ctx, "swiglu kernel");
 }
 
 }  // namespace

@@ -75,6 +75,15 @@ __device__ __forceinline__ void tma_load_4d_pair(uint32_t dst, const void *map, 
                  "l"(map), "r"(x), "r"(y), "r"(z), "r"(w), "r"(bar)
                  : "memory");
 }
+// The same by a CTA of its own, and the box asked into L2 only.
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const void *map, int x, int y, int z, int w, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst),
+                 "l"(map), "r"(x), "r"(y), "r"(z), "r"(w), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void tma_prefetch_4d(const void *map, int x, int y, int z, int w) {
+    asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];" ::"l"(map), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
 __device__ __forceinline__ void prefetch_tensormap(const void *map) { asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory"); }
 
 }  // namespace dev
