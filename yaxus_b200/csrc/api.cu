@@ -285,6 +285,10 @@ int attend_impl(yx_ctx *ctx, yx_kv *kv, int layer, const void *q, int q_dtype, i
     DeviceGuard guard(ctx->device);
 
     const int path = pick_path(ctx, kv);
+    // f32 caches: where some sequence brings more than 16 queries to a KV head, tiles of keys shared by up to 64 of them.
+    // One row a sequence is better off with the kernel that takes a row at a time (12 sequences of 600 to 2500 keys, two
+    // layers: 108 us there, 125 us here), and asking for path 1 gets that kernel.
+    const bool f32_tiles = path == 1 && kv->dtype == YX_F32 && ctx->tuning.force_path != 1 && (uint64_t)ctx->pass.longest_run * group > 16;
     const int64_t launches0 = ctx->launches;
     PlanParams pp{};
     pp.hkv = kv->hkv;
@@ -293,7 +297,7 @@ int attend_impl(yx_ctx *ctx, yx_kv *kv, int layer, const void *q, int q_dtype, i
     pp.key_lo = key_lo;
     pp.key_hi = key_hi;
     pp.esize = kv->esize;
-    const int per_sm = ctx->tuning.ctas_per_sm > 0 ? ctx->tuning.ctas_per_sm : (path == 1 ? 4 : 1);
+    const int per_sm = ctx->tuning.ctas_per_sm > 0 ? ctx->tuning.ctas_per_sm : (path == 1 ? (f32_tiles ? 2 : 4) : 1);
     pp.n_ctas = ctx->sm_count * per_sm;
     // The tensor split-key kernel is planned for one CTA fewer than there are SMs unless the
     // tuning asks for a count.  These calls run back to back, each one's grid launched while the
@@ -303,10 +307,10 @@ int attend_impl(yx_ctx *ctx, yx_kv *kv, int layer, const void *q, int q_dtype, i
     // the number of CTAs).  With an SM spare one CTA of the call behind always runs a call ahead.
     if (path == 2 && ctx->tuning.ctas_per_sm <= 0 && pp.n_ctas > 1) pp.n_ctas -= 1;
     // (a slot of the split-key kernel holds 32 query rows of f32 or 64 of a 16-bit type)
-    pp.max_rows = path == 1 ? 1 : std::max(1, std::min(MAX_ITEM_ROWS, (q_dtype == YX_F32 ? 32 : 64) / group));
-    pp.share_prefix = path != 1 && ctx->tuning.share_prefix != 2;
-    pp.w32 = ctx->tuning.cost32 > 0 ? ctx->tuning.cost32 : 16;
-    pp.w64 = ctx->tuning.cost64 > 0 ? ctx->tuning.cost64 : 40;
+    pp.max_rows = path == 1 && !f32_tiles ? 1 : std::max(1, std::min(MAX_ITEM_ROWS, (q_dtype == YX_F32 && !f32_tiles ? 32 : 64) / group));
+    pp.share_prefix = (path != 1 || f32_tiles) && ctx->tuning.share_prefix != 2;
+    pp.w32 = ctx->tuning.cost32 > 0 ? ctx->tuning.cost32 : (f32_tiles ? 24 : 16);
+    pp.w64 = ctx->tuning.cost64 > 0 ? ctx->tuning.cost64 : (f32_tiles ? 44 : 40);
     pp.resolve = path == 2;
     pp.share_rows = ctx->tuning.share_rows;
     // Prompt-sized runs of rows on a 16-bit cache go to the tcgen05 kernel; it writes final
@@ -318,7 +322,7 @@ int attend_impl(yx_ctx *ctx, yx_kv *kv, int layer, const void *q, int q_dtype, i
     pp.tile_ctas = ctx->sm_count;
     pp.tile_pairs = group % 2 == 0 && !(kv->dtype == YX_BF16 && q_dtype == YX_F32) && ctx->tuning.tile_single != 1;
     pp.min_piece = ctx->tuning.min_piece > 0 ? ctx->tuning.min_piece : (path == 2 ? 2 : 1);
-    pp.item_cost = ctx->tuning.item_cost > 0 ? ctx->tuning.item_cost - 1 : (path == 2 ? 14 : 0);
+    pp.item_cost = ctx->tuning.item_cost > 0 ? ctx->tuning.item_cost - 1 : (path == 2 ? 14 : (f32_tiles ? 12 : 0));
     // (taken before get_plan, whose upload of a new plan is itself an ordering point on the stream)
     const bool predecessor_is_split_key_call = ctx->last_launch == yx_ctx::LAST_SPLIT_KEY;
     const bool predecessor_wrote_marked_tiles_only =
@@ -465,7 +469,7 @@ int attend_impl(yx_ctx *ctx, yx_kv *kv, int layer, const void *q, int q_dtype, i
         profile_mark(ctx, 3);
     } else {
         if (!pl.items.empty())
-            if (int rc = launch_attend_simt(ctx, a)) return rc;
+            if (int rc = f32_tiles ? launch_attend_f32(ctx, a) : launch_attend_simt(ctx, a)) return rc;
         profile_mark(ctx, 1);
         profile_mark(ctx, 2);
         if (need_combine)
@@ -774,13 +778,15 @@ int yx_begin_pass(yx_ctx *ctx, uint32_t rows, const uint32_t *pos, const uint32_
     if (rows && (!pos || !kv_slot || !pt_off)) return fail(ctx, YX_ERR_INVALID, "begin_pass: null array");
     if (n_pages && !pages) return fail(ctx, YX_ERR_INVALID, "begin_pass: null page table");
     if (rows > 65535) return fail(ctx, YX_ERR_UNSUPPORTED, "begin_pass: more than 65535 rows");
-    uint32_t max_pos = 0, max_slot = 0, max_page = 0;
+    uint32_t max_pos = 0, max_slot = 0, max_page = 0, run = 0, longest_run = 0;
     for (uint32_t r = 0; r < rows; r++) {
         if ((uint64_t)pt_off[r] + pos[r] / PAGE >= n_pages)
             return fail(ctx, YX_ERR_INVALID, "begin_pass: a row's page table runs past `pages`");
         // kv_slot must be the slot of the row's own position (PassMeta, lib.rs:69-70).
         if (kv_slot[r] != pages[pt_off[r] + pos[r] / PAGE] * (uint32_t)PAGE + pos[r] % PAGE)
             return fail(ctx, YX_ERR_INVALID, "begin_pass: kv_slot is not slot(pages, pos)");
+        run = r > 0 && pt_off[r] == pt_off[r - 1] ? run + 1 : 1;
+        longest_run = std::max(longest_run, run);
         max_pos = std::max(max_pos, pos[r]);
         max_slot = std::max(max_slot, kv_slot[r]);
     }
@@ -795,6 +801,7 @@ int yx_begin_pass(yx_ctx *ctx, uint32_t rows, const uint32_t *pos, const uint32_
     p.max_pos_seen = max_pos;
     p.max_slot_seen = max_slot;
     p.max_page_seen = max_page;
+    p.longest_run = longest_run;
     ctx->pass_serial++;
     ctx->have_pass = true;
 

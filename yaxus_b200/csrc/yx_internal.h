@@ -182,6 +182,7 @@ struct PassHost {
     uint32_t max_pos_seen = 0;    // largest position of a row
     uint32_t max_page_seen = 0;   // largest page id in `pages`
     uint32_t max_slot_seen = 0;   // largest kv_slot of a row
+    uint32_t longest_run = 0;     // most rows in a row with one page table
 };
 
 struct PlanParams {
@@ -440,6 +441,7 @@ struct TileArgs {
 };
 int launch_prefill_tc(yx_ctx *ctx, const TileArgs &a);
 int launch_attend_simt(yx_ctx *ctx, const AttendArgs &a);
+int launch_attend_f32(yx_ctx *ctx, const AttendArgs &a);
 int launch_attend_mma(yx_ctx *ctx, const AttendArgs &a);
 // Writes the empty mark (-1e30, 0, 0) for n (row, head) triples.
 int launch_fill_empty(yx_ctx *ctx, size_t n, float *m, float *l, float *o);
