@@ -347,8 +347,8 @@ int attend_impl(yx_ctx *ctx, yx_kv *kv, int layer, const void *q, int q_dtype, i
     ctx->ws_set ^= 1;
     float *const part_o = ctx->ws_o + (size_t)ctx->ws_set * (o_bytes / sizeof(float));
     float *const part_ml = ctx->ws_ml + (size_t)ctx->ws_set * (ml_bytes / sizeof(float));
-    if (path == 2) {
-        // Arrival counters of the fused merge: zero when allocated, and every launch leaves
+    if (!f32_tiles) {
+        // Arrival counters of the fused merges: zero when allocated, and every launch leaves
         // them zero again.
         size_t need = (size_t)ctx->pass.rows * kv->hkv * sizeof(uint32_t);
         if (need > ctx->counters_cap || !ctx->counters) {
@@ -468,11 +468,14 @@ int attend_impl(yx_ctx *ctx, yx_kv *kv, int layer, const void *q, int q_dtype, i
         host_clock_lap(ctx, 6);
         profile_mark(ctx, 3);
     } else {
+        // (rows without a live key in the range get no item, so the merge inside the row kernel does not write them)
+        if (!f32_tiles && o_out && pl.has_empty_rows)
+            if (int rc = launch_fill_empty(ctx, (size_t)ctx->pass.rows * hq, m_out, l_out, o_out)) return rc;
         if (!pl.items.empty())
-            if (int rc = f32_tiles ? launch_attend_f32(ctx, a) : launch_attend_simt(ctx, a)) return rc;
+            if (int rc = f32_tiles ? launch_attend_f32(ctx, a) : launch_attend_simt(ctx, a, cp->d_merges)) return rc;
         profile_mark(ctx, 1);
         profile_mark(ctx, 2);
-        if (need_combine)
+        if (f32_tiles && need_combine)
             if (int rc = launch_combine(ctx, cp->d_merges, part_o, part_ml, (int)ctx->pass.rows, hq, group, out,
                                         out_dtype, m_out, l_out, o_out))
                 return rc;

@@ -8,11 +8,15 @@
 // them in flight;
 // a lane holds four of the 128 dims, so a K or V row is one coalesced 512-byte (f32) or
 // 256-byte (16-bit) read per warp; the four warps' triples are merged in shared memory.
-// K and V are read straight from global memory: each byte is used once per head chunk.
+// K and V are read straight from global memory: each byte is used once per head chunk.  The parts of a row are
+// merged by whichever of its CTAs comes last, without a launch of their own.
+// Bound by issue slots and latencies, not yet by HBM: twelve sequences of 600 to 2500 keys on 4 f32 KV heads (77 MB)
+// take 31 us, launch and merge included, where separate sums over the warp for every key and head and a merge kernel
+// took 28 + 9 us with twice the exchanges (two layers: 109 -> 84 us); one sequence of 1024 keys 49 -> 43 us.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
-#include "yx_internal.h"
+#include "yx_device.cuh"
 
 namespace yx {
 namespace {
@@ -49,14 +53,77 @@ __device__ __forceinline__ float4 load_q4(const void *q, int q_dtype, size_t ele
     return make_float4(a.x, a.y, b.x, b.y);
 }
 
-__global__ void __launch_bounds__(WARPS * 32)
+// The lanes whose bit `bit` is clear get a + their partner's a, the others b + their partner's b.
+__device__ __forceinline__ float halve(float a, float b, int bit, int lane) {
+    const bool upper = (lane & bit) != 0;
+    return (upper ? b : a) + __shfl_xor_sync(0xffffffffu, upper ? a : b, bit);
+}
+// Where a call's merged rows go (any of out and the triple's three may be null), and what the merge needs.
+struct RowMerge {
+    const Merge *merges;
+    uint32_t *counters;      // one per (row, KV head), zero between launches
+    void *out;
+    int out_dtype;
+    float *m, *l, *o;
+};
+
+// The merge of combine.cu for one (row, query head), by a warp: lane c weighs part c, then all of them are added up in
+// order, eight vectors asked for at once.  Every part of this kernel has been written, so empty ones (l <= 0) may be
+// read; they are left out by their weight, whatever they hold.
+__device__ __forceinline__ void merge_parts(const RowMerge &fin, const Merge &mg, const float *part_o, const float *part_ml, int g, int group,
+                                            size_t idx, int lane) {
+    float mx = -1e30f, l = 0.0f;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (uint32_t c0 = 0; c0 < mg.count; c0 += 32) {
+        const uint32_t nc = min(32u, mg.count - c0);
+        float2 ml = make_float2(-1e30f, 0.0f);
+        if ((uint32_t)lane < nc) ml = __ldcg((const float2 *)(part_ml + ((size_t)(mg.first + c0 + lane) * group + g) * 2));
+        const bool live = ml.y > 0.0f;
+        float cm = live ? ml.x : -1e30f;
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) cm = fmaxf(cm, __shfl_xor_sync(0xffffffffu, cm, off));
+        const float nm = fmaxf(mx, cm), r = __expf(mx - nm), w = live ? __expf(ml.x - nm) : 0.0f;
+        float ls = live ? ml.y * w : 0.0f;
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) ls += __shfl_xor_sync(0xffffffffu, ls, off);
+        l = l * r + ls;
+        acc = make_float4(acc.x * r, acc.y * r, acc.z * r, acc.w * r);
+        mx = nm;
+        for (uint32_t j0 = 0; j0 < nc; j0 += 8) {
+            float4 po[8];
+#pragma unroll
+            for (uint32_t j = 0; j < 8; j++)
+                po[j] = j0 + j < nc ? __ldcg((const float4 *)(part_o + ((size_t)(mg.first + c0 + j0 + j) * group + g) * D + lane * 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (uint32_t j = 0; j < 8; j++) {
+                const float wj = __shfl_sync(0xffffffffu, w, (int)((j0 + j) & 31u));
+                if (j0 + j < nc && wj != 0.0f) acc = make_float4(acc.x + po[j].x * wj, acc.y + po[j].y * wj, acc.z + po[j].z * wj, acc.w + po[j].w * wj);
+            }
+        }
+    }
+    if (fin.out) {
+        const float inv = 1.0f / l;   // a row always sees its own key, so l > 0 for whole attention
+        dev::store4(fin.out, fin.out_dtype, idx * D + lane * 4, make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv));
+    }
+    if (fin.o) {
+        *(float4 *)(fin.o + idx * D + lane * 4) = acc;
+        if (lane == 0) {
+            fin.m[idx] = mx;
+            fin.l[idx] = l;
+        }
+    }
+}
+static_assert(HC == 4 && KU == 8, "a lane ends up with one of 8 keys x 4 heads");
+
+__global__ void __launch_bounds__(WARPS * 32, 4)
 attend_simt_kernel(const void *__restrict__ q, int q_dtype, int hq, int group, const char *__restrict__ k_arena,
                    const char *__restrict__ v_arena, int hkv, int kv_dtype, uint32_t kv_pages, uint32_t window,
                    const uint32_t *__restrict__ pos, const uint32_t *__restrict__ pages, const Item *__restrict__ items,
-                   const uint32_t *__restrict__ cta_begin, float *__restrict__ part_o, float *__restrict__ part_ml,
-                   yx_dev_status *status) {
+                   const uint32_t *__restrict__ cta_begin, float *part_o, float *part_ml, const RowMerge fin, yx_dev_status *status) {
     __shared__ float sm_o[WARPS][HC][D];
     __shared__ float sm_ml[WARPS][HC][2];
+    __shared__ __align__(16) float sm_e[WARPS][KU + 1][HC];
+    __shared__ bool last;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const float scale = 0.08838834764831845f;   // 1 / sqrt(128), the reference's f32 value
     // A programmatic dependent of the kernel before it: resident while that kernel finishes, it
@@ -77,14 +144,12 @@ attend_simt_kernel(const void *__restrict__ q, int q_dtype, int hq, int group, c
             uint32_t k1 = min(min(p, it.key_hi), it.tile_end * TILE_KEYS - 1);   // inclusive
             for (int h0 = 0; h0 < group; h0 += HC) {
                 float4 qv[HC];
-                float m[HC], l[HC];
                 float4 o[HC];
+                float m = -INFINITY, l = 0.0f;   // of head h0 + lane / 8; l over the keys lane % 8 of every round
 #pragma unroll
                 for (int g = 0; g < HC; g++) {
                     int hh = min(h0 + g, group - 1);
                     qv[g] = load_q4(q, q_dtype, ((size_t)row * hq + kvh * group + hh) * D + lane * 4);
-                    m[g] = -INFINITY;
-                    l[g] = 0.0f;
                     o[g] = make_float4(0.f, 0.f, 0.f, 0.f);
                 }
                 // KU keys of this warp at a time: their page ids, then their K and V rows, are asked
@@ -99,6 +164,7 @@ attend_simt_kernel(const void *__restrict__ q, int q_dtype, int hq, int group, c
                         live[u] = key <= k1;
                         page[u] = live[u] ? pages[it.pt_off + (uint32_t)(key / PAGE)] : 0u;
                     }
+                    uint32_t dead = 0;   // keys of the round that do not count
 #pragma unroll
                     for (int u = 0; u < KU; u++) {
                         const uint64_t key = key0 + (uint64_t)u * WARPS;
@@ -115,41 +181,68 @@ attend_simt_kernel(const void *__restrict__ q, int q_dtype, int hq, int group, c
                             const int tok = (int)(key % PAGE);
                             kk[u] = load4(k_arena, kv_dtype, page[u], hkv, kvh, tok, lane);
                             vv[u] = load4(v_arena, kv_dtype, page[u], hkv, kvh, tok, lane);
+                        } else {
+                            dead |= 1u << u;
                         }
+                    }
+                    // KU x HC dot products over 32 lanes end with one in each lane, key lane % 8 of head lane / 8: at
+                    // every step a lane hands half of what it holds to its partner and keeps the other half, 31 exchanges
+                    // where a sum of each over all lanes takes 160.
+                    float s[KU];
+#pragma unroll
+                    for (int u = 0; u < KU; u++) {
+                        float d[HC];
+#pragma unroll
+                        for (int g = 0; g < HC; g++)
+                            d[g] = qv[g].x * kk[u].x + qv[g].y * kk[u].y + qv[g].z * kk[u].z + qv[g].w * kk[u].w;
+                        const float a = halve(d[0], d[2], 16, lane), b = halve(d[1], d[3], 16, lane);
+                        s[u] = halve(a, b, 8, lane);
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; u++) s[u] = halve(s[u], s[u + 4], 4, lane);
+                    s[0] = halve(s[0], s[2], 2, lane);
+                    s[1] = halve(s[1], s[3], 2, lane);
+                    const float sc = halve(s[0], s[1], 1, lane) * scale;
+                    const bool counts = ((dead >> (lane & 7)) & 1u) == 0;
+                    float mx = counts ? sc : -INFINITY;
+#pragma unroll
+                    for (int off = 4; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+                    const float mn = fmaxf(m, mx);
+                    const float f = m == -INFINITY ? 0.0f : exp2f((m - mn) * LOG2E);
+                    const float e = counts ? exp2f((sc - mn) * LOG2E) : 0.0f;
+                    l = l * f + e;
+                    m = mn;
+                    // Back to every lane through shared memory: [key][head], the rescales behind them.
+                    __syncwarp();
+                    sm_e[warp][lane & 7][lane >> 3] = e;
+                    if ((lane & 7) == 0) sm_e[warp][KU][lane >> 3] = f;
+                    __syncwarp();
+                    {
+                        const float4 fs = *(const float4 *)sm_e[warp][KU];
+                        const float fg[HC] = {fs.x, fs.y, fs.z, fs.w};
+#pragma unroll
+                        for (int g = 0; g < HC; g++) o[g] = make_float4(o[g].x * fg[g], o[g].y * fg[g], o[g].z * fg[g], o[g].w * fg[g]);
                     }
 #pragma unroll
                     for (int u = 0; u < KU; u++) {
-                        if (!live[u]) continue;   // (uniform over the warp)
-                        float s[HC];
-#pragma unroll
-                        for (int g = 0; g < HC; g++)
-                            s[g] = qv[g].x * kk[u].x + qv[g].y * kk[u].y + qv[g].z * kk[u].z + qv[g].w * kk[u].w;
-#pragma unroll
-                        for (int off = 16; off > 0; off >>= 1)
-#pragma unroll
-                            for (int g = 0; g < HC; g++) s[g] += __shfl_xor_sync(0xffffffffu, s[g], off);
+                        const float4 es = *(const float4 *)sm_e[warp][u];
+                        const float eg[HC] = {es.x, es.y, es.z, es.w};
 #pragma unroll
                         for (int g = 0; g < HC; g++) {
-                            float sc = s[g] * scale;
-                            float mn = fmaxf(m[g], sc);
-                            float a = exp2f((m[g] - mn) * LOG2E);   // 0 on the first key (m = -inf)
-                            float e = exp2f((sc - mn) * LOG2E);
-                            l[g] = l[g] * a + e;
-                            o[g].x = o[g].x * a + e * vv[u].x;
-                            o[g].y = o[g].y * a + e * vv[u].y;
-                            o[g].z = o[g].z * a + e * vv[u].z;
-                            o[g].w = o[g].w * a + e * vv[u].w;
-                            m[g] = mn;
+                            o[g].x += eg[g] * vv[u].x;
+                            o[g].y += eg[g] * vv[u].y;
+                            o[g].z += eg[g] * vv[u].z;
+                            o[g].w += eg[g] * vv[u].w;
                         }
                     }
                 }
 #pragma unroll
-                for (int g = 0; g < HC; g++) {
-                    *(float4 *)&sm_o[warp][g][lane * 4] = o[g];
-                    if (lane == 0) {
-                        sm_ml[warp][g][0] = m[g];
-                        sm_ml[warp][g][1] = l[g];
-                    }
+                for (int off = 4; off > 0; off >>= 1) l += __shfl_xor_sync(0xffffffffu, l, off);
+#pragma unroll
+                for (int g = 0; g < HC; g++) *(float4 *)&sm_o[warp][g][lane * 4] = o[g];
+                if ((lane & 7) == 0) {
+                    sm_ml[warp][lane >> 3][0] = m;
+                    sm_ml[warp][lane >> 3][1] = l;
                 }
                 __syncthreads();
                 // Thread t merges dim t of the four warps' triples, head by head.
@@ -169,41 +262,39 @@ attend_simt_kernel(const void *__restrict__ q, int q_dtype, int hq, int group, c
                         acc += sm_o[w][g][t] * f;
                     }
                     size_t slot = (size_t)it.part[r] * group + h0 + g;
-                    part_o[slot * D + t] = acc;
-                    if (t == 0) {
-                        // An item without a live key for this row: the reference's empty mark.
-                        part_ml[slot * 2] = mx == -INFINITY ? -1e30f : mx;
-                        part_ml[slot * 2 + 1] = ls;
-                    }
+                    __stcg(part_o + slot * D + t, acc);
+                    // An item without a live key for this row: the reference's empty mark.
+                    if (t == 0) __stcg((float2 *)(part_ml + slot * 2), make_float2(mx == -INFINITY ? -1e30f : mx, ls));
                 }
                 __syncthreads();
             }
+            if (!fin.merges) continue;   // (measurement hook)
+            // The last of a row and KV head's parts to be written merges them all, a warp to a query head.
+            const Merge mg = fin.merges[(size_t)row * hkv + kvh];
+            __threadfence();
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                uint32_t *counter = fin.counters + (size_t)row * hkv + kvh;
+                last = mg.count == 1 || atomicAdd(counter, 1u) == mg.count - 1;
+                if (last && mg.count > 1) *counter = 0u;
+            }
+            __syncthreads();
+            if (last) {
+                __threadfence();
+                for (int g = warp; g < group; g += WARPS) merge_parts(fin, mg, part_o, part_ml, g, group, (size_t)row * hq + kvh * group + g, lane);
+            }
+            __syncthreads();   // (`last` is the next row's)
         }
     }
 }
 
 }  // namespace
 
-int launch_attend_simt(yx_ctx *ctx, const AttendArgs &a) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)a.n_ctas);
-    cfg.blockDim = dim3(WARPS * 32);
-    cfg.stream = ctx->stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    const uint32_t window = (uint32_t)std::max<int64_t>(a.window, 0);
-    if (int rc = check_cuda(ctx,
-                            cudaLaunchKernelEx(&cfg, attend_simt_kernel, a.q, a.q_dtype, a.hq, a.group, (const char *)a.k_arena,
-                                               (const char *)a.v_arena, a.hkv, a.kv_dtype, a.kv_pages, window,
-                                               (const uint32_t *)ctx->d_pos, (const uint32_t *)ctx->d_pages, a.items, a.cta_begin,
-                                               a.part_o, a.part_ml, ctx->dev_status),
-                            "attend_simt kernel launch"))
-        return rc;
-    ctx->launches++;
-    return check_cuda(ctx, cudaGetLastError(), "attend_simt kernel");
+int launch_attend_simt(yx_ctx *ctx, const AttendArgs &a, const Merge *merges) {
+    const RowMerge fin{ctx->skip_merge ? nullptr : merges, a.counters, a.out, a.out_dtype, a.m_out, a.l_out, a.o_out};
+    return launch_dependent(ctx, "attend_simt kernel launch", attend_simt_kernel, dim3((unsigned)a.n_ctas), dim3(WARPS * 32), 0, a.q, a.q_dtype,
+                            a.hq, a.group, a.k_arena, a.v_arena, a.hkv, a.kv_dtype, a.kv_pages, (uint32_t)std::max<int64_t>(a.window, 0),
+                            ctx->d_pos, ctx->d_pages, a.items, a.cta_begin, a.part_o, a.part_ml, fin, ctx->dev_status);
 }
 
 }  // namespace yx

@@ -440,7 +440,7 @@ struct TileArgs {
     const uint32_t *wide_v;  // the cache's "V holds values f16 cannot" flag (device)
 };
 int launch_prefill_tc(yx_ctx *ctx, const TileArgs &a);
-int launch_attend_simt(yx_ctx *ctx, const AttendArgs &a);
+int launch_attend_simt(yx_ctx *ctx, const AttendArgs &a, const Merge *merges);   // merges too
 int launch_attend_f32(yx_ctx *ctx, const AttendArgs &a);
 int launch_attend_mma(yx_ctx *ctx, const AttendArgs &a);
 // Writes the empty mark (-1e30, 0, 0) for n (row, head) triples.
