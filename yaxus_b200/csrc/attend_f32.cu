@@ -14,7 +14,9 @@
 // them there, two tiles in flight.
 //
 // Bound by the latencies of its own arithmetic at two warps a scheduler (FMA pipe half busy), not by memory.  A
-// 1000-row prompt behind 1000 keys, 16 query / 4 KV heads, two layers: a whole step 5415 -> 1349 us.
+// 1000-row prompt behind 1000 keys, 16 query / 4 KV heads, two layers: a whole step 5415 -> 1385 us.
+// Sums are blocked by 32 dims and 32 keys, which costs 36 us of that: the error against 64 bits over 300 rows behind
+// 1000 keys is 2.0e-7 with it, 4.0e-7 without, and 3.3e-7 for the kernel that takes a row at a time.
 #include <type_traits>
 
 #include "yx_device.cuh"
@@ -62,6 +64,11 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
 __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
     uint64_t d;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
 __device__ __forceinline__ uint64_t both(float x) {
@@ -168,31 +175,40 @@ __device__ __forceinline__ void run_item(const Params &P, const Item &it, Shared
         }
         const float *k = s_kv + stage * 2 * TILE_FLOATS, *v = k + TILE_FLOATS;
         if (!sh.bad_page[stage]) {   // (uniform over the CTA)
-            // Scores of RT rows against keys tx and tx + 16: even dims in one half of the pair, odd ones in the other.
+            // Scores of RT rows against keys tx and tx + 16: even dims in one half of the pair, odd ones in the other, 32 dims
+            // at a time, so that no chain of rounded sums is longer than 16.
             uint64_t s2[RT][2];
+#pragma unroll 1
+            for (int d0 = 0; d0 < D; d0 += 32) {
+                uint64_t part[RT][2];
 #pragma unroll
-            for (int r = 0; r < RT; r++) s2[r][0] = s2[r][1] = 0ull;
-#pragma unroll 4
-            for (int d = 0; d < D; d += 4) {
-                const ulonglong2 ka = *(const ulonglong2 *)(k + tx * STRIDE + d), kb = *(const ulonglong2 *)(k + (tx + 16) * STRIDE + d);
-                uint64_t q_hi[RT];
+                for (int d = 0; d < 32; d += 4) {
+                    const ulonglong2 ka = *(const ulonglong2 *)(k + tx * STRIDE + d0 + d), kb = *(const ulonglong2 *)(k + (tx + 16) * STRIDE + d0 + d);
+                    uint64_t q_hi[RT];
 #pragma unroll
-                for (int r = 0; r < RT; r++) {
-                    const ulonglong2 qv = *(const ulonglong2 *)(q_rows + r * STRIDE + d);
-                    s2[r][0] = fma2(qv.x, ka.x, s2[r][0]);
-                    s2[r][1] = fma2(qv.x, kb.x, s2[r][1]);
-                    q_hi[r] = qv.y;
+                    for (int r = 0; r < RT; r++) {
+                        const ulonglong2 qv = *(const ulonglong2 *)(q_rows + r * STRIDE + d0 + d);
+                        part[r][0] = d == 0 ? mul2(qv.x, ka.x) : fma2(qv.x, ka.x, part[r][0]);
+                        part[r][1] = d == 0 ? mul2(qv.x, kb.x) : fma2(qv.x, kb.x, part[r][1]);
+                        q_hi[r] = qv.y;
+                    }
+                    // (the other two dims only now: back to back, each would wait for the sum before it)
+#pragma unroll
+                    for (int r = 0; r < RT; r++) {
+                        part[r][0] = fma2(q_hi[r], ka.y, part[r][0]);
+                        part[r][1] = fma2(q_hi[r], kb.y, part[r][1]);
+                    }
                 }
-                // (the other two dims only now: back to back, each would wait for the sum before it)
 #pragma unroll
                 for (int r = 0; r < RT; r++) {
-                    s2[r][0] = fma2(q_hi[r], ka.y, s2[r][0]);
-                    s2[r][1] = fma2(q_hi[r], kb.y, s2[r][1]);
+                    s2[r][0] = d0 == 0 ? part[r][0] : add2(s2[r][0], part[r][0]);
+                    s2[r][1] = d0 == 0 ? part[r][1] : add2(s2[r][1], part[r][1]);
                 }
             }
             // Every key of the tile live for every query: no masks.
             const bool edge = t * KEYS < sh.all_from || t * KEYS + KEYS - 1 > sh.all_to;
             const uint32_t key_a = t * KEYS + tx, key_b = key_a + 16;
+            float rescale[RT];
 #pragma unroll
             for (int r = 0; r < RT; r++) {
                 const float2 a = halves(s2[r][0]), b = halves(s2[r][1]);
@@ -211,16 +227,18 @@ __device__ __forceinline__ void run_item(const Params &P, const Item &it, Shared
                 const float ea = live_a ? exp2f((sa - mn) * LOG2E) : 0.0f, eb = live_b ? exp2f((sb - mn) * LOG2E) : 0.0f;
                 m[r] = mn;
                 l[r] = l[r] * f + (ea + eb);
-                const uint64_t ff = both(f);
-#pragma unroll
-                for (int c = 0; c < 4; c++) o[r][c] = mul2(o[r][c], ff);
+                rescale[r] = f;
                 // (a masked key is marked, so that its V row, which may hold anything, is left out altogether)
                 p_rows[r * P_STRIDE + tx] = live_a ? ea : -1.0f;
                 p_rows[r * P_STRIDE + tx + 16] = live_b ? eb : -1.0f;
             }
             __syncwarp();
+            // The tile's outputs are summed by themselves and then added to the rescaled ones before: chains of 32 keys.
             auto products = [&](auto masked) {
-#pragma unroll 2
+                uint64_t sum[RT][4];
+#pragma unroll
+                for (int r = 0; r < RT; r++) sum[r][0] = sum[r][1] = sum[r][2] = sum[r][3] = 0ull;
+#pragma unroll 1
                 for (int k4 = 0; k4 < KEYS; k4 += 4) {
                     float p[RT][4];
 #pragma unroll
@@ -232,12 +250,18 @@ __device__ __forceinline__ void run_item(const Params &P, const Item &it, Shared
                         for (int r = 0; r < RT; r++) {
                             if (decltype(masked)::value && p[r][j] < 0.0f) continue;
                             const uint64_t pp = both(p[r][j]);
-                            o[r][0] = fma2(pp, va.x, o[r][0]);
-                            o[r][1] = fma2(pp, va.y, o[r][1]);
-                            o[r][2] = fma2(pp, vb.x, o[r][2]);
-                            o[r][3] = fma2(pp, vb.y, o[r][3]);
+                            sum[r][0] = fma2(pp, va.x, sum[r][0]);
+                            sum[r][1] = fma2(pp, va.y, sum[r][1]);
+                            sum[r][2] = fma2(pp, vb.x, sum[r][2]);
+                            sum[r][3] = fma2(pp, vb.y, sum[r][3]);
                         }
                     }
+                }
+#pragma unroll
+                for (int r = 0; r < RT; r++) {
+                    const uint64_t f = both(rescale[r]);
+#pragma unroll
+                    for (int c = 0; c < 4; c++) o[r][c] = fma2(o[r][c], f, sum[r][c]);
                 }
             };
             if (edge) products(std::true_type{});
