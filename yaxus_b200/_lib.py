@@ -42,6 +42,7 @@ class PlanInfo(ctypes.Structure):
 _U32P = POINTER(c_uint32)
 _F32P = POINTER(c_float)
 
+# Arrays of u32 are taken as addresses (an integer, or any pointer object).
 # name -> (restype, argtypes); exactly the functions include/yaxus_cuda.h declares.
 SIGNATURES = {
     "yx_ctx_create": (c_int, [c_int, c_void_p, POINTER(c_void_p)]),
@@ -67,19 +68,19 @@ SIGNATURES = {
     "yx_kv_copy_page": (c_int, [c_void_p, c_void_p, c_uint32, c_uint32]),
     "yx_kv_read_pages": (c_int, [c_void_p, c_void_p, c_int, c_uint32, c_uint32, c_void_p, c_void_p]),
     "yx_kv_write_pages": (c_int, [c_void_p, c_void_p, c_int, c_uint32, c_uint32, c_void_p, c_void_p]),
-    "yx_begin_pass": (c_int, [c_void_p, c_uint32, _U32P, _U32P, _U32P, _U32P, c_uint32]),
+    "yx_begin_pass": (c_int, [c_void_p, c_uint32, c_void_p, c_void_p, c_void_p, c_void_p, c_uint32]),
     "yx_attention": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_float, c_void_p]),
     "yx_kv_append": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int]),
     "yx_attend": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int64, c_void_p, c_int]),
-    "yx_embed": (c_int, [c_void_p, c_void_p, c_uint32, c_uint32, _U32P, c_uint32, c_void_p]),
+    "yx_embed": (c_int, [c_void_p, c_void_p, c_uint32, c_uint32, c_void_p, c_uint32, c_void_p]),
     "yx_rmsnorm": (c_int, [c_void_p, c_void_p, c_void_p, c_uint32, c_uint32, c_float, c_float, c_void_p]),
     "yx_add_norm": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_float, c_float, c_uint32, c_uint32, c_void_p]),
     "yx_matmul": (c_int, [c_void_p, c_void_p, c_void_p, c_uint32, c_uint32, c_uint32, c_void_p]),
     "yx_matmul_glu": (c_int, [c_void_p, c_void_p, c_void_p, c_uint32, c_uint32, c_uint32, c_void_p]),
     "yx_swiglu": (c_int, [c_void_p, c_void_p, c_uint32, c_uint32, c_void_p]),
     "yx_add_assign": (c_int, [c_void_p, c_void_p, c_void_p, c_size_t]),
-    "yx_select_rows": (c_int, [c_void_p, c_void_p, c_uint32, c_uint32, _U32P, c_uint32, c_void_p]),
-    "yx_argmax_rows": (c_int, [c_void_p, c_void_p, c_uint32, c_uint32, _U32P]),
+    "yx_select_rows": (c_int, [c_void_p, c_void_p, c_uint32, c_uint32, c_void_p, c_uint32, c_void_p]),
+    "yx_argmax_rows": (c_int, [c_void_p, c_void_p, c_uint32, c_uint32, c_void_p]),
     "yx_attend_static": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int64, c_void_p, c_int]),
     "yx_attend_partial": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int64, c_uint64, c_uint64,
                                   c_void_p, c_void_p, c_void_p]),

@@ -75,16 +75,21 @@ class Kv:
             pass
 
 
+# Addresses go to the C ABI as plain integers: at decode sizes an operator's kernel takes no longer than
+# its call, and making a ctypes object for every argument (2 us for a numpy array's) was a tenth of it.
 def _ptr(t: Optional[torch.Tensor]):
-    return ctypes.c_void_p(t.data_ptr()) if t is not None else None
+    return t.data_ptr() if t is not None else None
 
 
 def _u32(a) -> np.ndarray:
     return np.ascontiguousarray(a, dtype=np.uint32)
 
 
-def _u32p(a: np.ndarray):
-    return a.ctypes.data_as(ctypes.POINTER(ctypes.c_uint32))
+def _u32p(a: np.ndarray) -> int:
+    try:
+        return ctypes.addressof(ctypes.c_char.from_buffer(a))
+    except (TypeError, ValueError):   # read-only or empty
+        return a.ctypes.data
 
 
 class CudaBackend:
@@ -303,9 +308,9 @@ class CudaBackend:
         rows = qkv.shape[0]
         if rows != self._rows:   # the reference asserts this (cpu lib.rs:525)
             raise AssertionError("attention rows differ from the pass")
-        out = torch.empty(rows, hq * HEAD_DIM, dtype=torch.float32, device=self.device)
-        self._L.yx_attention(self._ctx, kv._h, layer.index, _ptr(qkv), _ptr(q_norm.float().contiguous()),
-                             _ptr(k_norm.float().contiguous()), hq, eps, _ptr(out))
+        q_norm, k_norm = q_norm.float().contiguous(), k_norm.float().contiguous()   # (named: alive until the launch is queued)
+        out = self._f32(rows, hq * HEAD_DIM)
+        self._L.yx_attention(self._ctx, kv._h, layer.index, _ptr(qkv), _ptr(q_norm), _ptr(k_norm), hq, eps, _ptr(out))
         return out
 
     # ---- the two halves of attention, for callers that hold final q, k, v ----------------
