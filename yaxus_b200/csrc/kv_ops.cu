@@ -67,10 +67,15 @@ __global__ void append_kernel(const void *__restrict__ k_rows, const void *__res
 }
 
 // write_rows (crates/yaxus-backend-cpu/src/lib.rs:359-385) ≡ qk_rope
-// (crates/yaxus-backend-gpu/src/shaders.rs:285-341).  One warp per (row, head) over the
-// hq + 2*hkv heads of a qkv row.  Lane l holds dims {2l, 2l+1, 2l+64, 2l+65}: both members of
+// (crates/yaxus-backend-gpu/src/shaders.rs:285-341).  One warp per HEADS of the hq + 2*hkv heads
+// of a qkv row.  Lane l holds dims {2l, 2l+1, 2l+64, 2l+65}: both members of
 // two rotation pairs.  cos/sin follow crates/yaxus-model/src/config.rs:213-219: f32 angle,
-// f64 cos/sin, f32 result times the concentration.
+// f64 cos/sin, f32 result times the concentration; they depend on the row alone, so a warp with
+// several heads takes them once.
+//
+// Prompts are bound by HBM once the 64-bit cosines are out of the way, decode steps by one warp's latency:
+// eight heads a warp where that still leaves every SM warps enough (see launch_qk_rope_append), one elsewhere.
+template <int HEADS>
 __global__ void qk_rope_append_kernel(const float *__restrict__ qkv, const float *__restrict__ q_norm,
                                       const float *__restrict__ k_norm, const uint32_t *__restrict__ pos,
                                       const uint32_t *__restrict__ kv_slot, uint32_t rows, int hq, int hkv,
@@ -78,59 +83,73 @@ __global__ void qk_rope_append_kernel(const float *__restrict__ qkv, const float
                                       char *__restrict__ k_arena, char *__restrict__ v_arena,
                                       float *__restrict__ q_out, uint32_t *__restrict__ wide_v) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // see append_kernel
-    const int heads = hq + 2 * hkv;
+    const int heads = hq + 2 * hkv, groups = (heads + HEADS - 1) / HEADS;
     uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int lane = threadIdx.x & 31;
-    if (warp >= rows * (uint32_t)heads) return;
-    uint32_t row = warp / (uint32_t)heads;
-    int head = (int)(warp % (uint32_t)heads);
-    const float *x = qkv + ((size_t)row * heads + head) * D;
-    float2 lo = *(const float2 *)(x + 2 * lane);
-    float2 hi = *(const float2 *)(x + 64 + 2 * lane);
-    const bool is_q = head < hq, is_k = !is_q && head < hq + hkv;
-    float r0 = lo.x, r1 = lo.y, r2 = hi.x, r3 = hi.y;
-    if (is_q || is_k) {
-        float ss = lo.x * lo.x + lo.y * lo.y + hi.x * hi.x + hi.y * hi.y;
+    if (warp >= rows * (uint32_t)groups) return;
+    const uint32_t row = warp / (uint32_t)groups;
+    const int head0 = (int)(warp % (uint32_t)groups) * HEADS;
+    const float *x = qkv + ((size_t)row * heads + head0) * D;
+    float2 lo[HEADS], hi[HEADS];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        float r = 1.0f / sqrtf(ss / (float)D + eps);
-        const float *w = is_q ? q_norm : k_norm;
-        float2 wl = *(const float2 *)(w + 2 * lane), wh = *(const float2 *)(w + 64 + 2 * lane);
-        // Separate roundings (no fused multiply-add), as in the reference's Rust arithmetic.
-        float a0 = __fmul_rn(1.0f + wl.x, __fmul_rn(lo.x, r)), a1 = __fmul_rn(1.0f + wl.y, __fmul_rn(lo.y, r));
-        float b0 = __fmul_rn(1.0f + wh.x, __fmul_rn(hi.x, r)), b1 = __fmul_rn(1.0f + wh.y, __fmul_rn(hi.y, r));
+    for (int h = 0; h < HEADS; h++) {
+        lo[h] = hi[h] = make_float2(0.f, 0.f);
+        if (head0 + h < heads) {
+            lo[h] = *(const float2 *)(x + h * D + 2 * lane);
+            hi[h] = *(const float2 *)(x + h * D + 64 + 2 * lane);
+        }
+    }
+    const uint32_t slot = kv_slot[row], page = slot / PAGE;
+    const int tok = (int)(slot % PAGE);
+    float c0 = 0.f, s0 = 0.f, c1 = 0.f, s1 = 0.f;
+    if (head0 < hq + hkv) {
         float p = (float)pos[row];
         float ang0 = __fmul_rn(p, rope->inv_freq[2 * lane]), ang1 = __fmul_rn(p, rope->inv_freq[2 * lane + 1]);
         float conc = rope->concentration;
-        float c0 = __fmul_rn((float)cos((double)ang0), conc), s0 = __fmul_rn((float)sin((double)ang0), conc);
-        float c1 = __fmul_rn((float)cos((double)ang1), conc), s1 = __fmul_rn((float)sin((double)ang1), conc);
-        r0 = __fsub_rn(__fmul_rn(a0, c0), __fmul_rn(b0, s0));
-        r2 = __fadd_rn(__fmul_rn(b0, c0), __fmul_rn(a0, s0));
-        r1 = __fsub_rn(__fmul_rn(a1, c1), __fmul_rn(b1, s1));
-        r3 = __fadd_rn(__fmul_rn(b1, c1), __fmul_rn(a1, s1));
+        c0 = __fmul_rn((float)cos((double)ang0), conc), s0 = __fmul_rn((float)sin((double)ang0), conc);
+        c1 = __fmul_rn((float)cos((double)ang1), conc), s1 = __fmul_rn((float)sin((double)ang1), conc);
     }
-    if (is_q) {
-        float *q = q_out + ((size_t)row * hq + head) * D;
-        *(float2 *)(q + 2 * lane) = make_float2(r0, r1);
-        *(float2 *)(q + 64 + 2 * lane) = make_float2(r2, r3);
-        return;
-    }
-    int h = is_k ? head - hq : head - hq - hkv;
-    char *arena = is_k ? k_arena : v_arena;
-    uint32_t slot = kv_slot[row];
-    uint32_t page = slot / PAGE;
-    int tok = (int)(slot % PAGE);
-    if (kv_dtype == YX_F32) {
-        float *d = (float *)arena + kv_off32(page, hkv, h, tok, 0);
-        *(float2 *)(d + 2 * lane) = make_float2(r0, r1);
-        *(float2 *)(d + 64 + 2 * lane) = make_float2(r2, r3);
-    } else {
-        uint32_t a = (uint32_t)to_storage(r0, kv_dtype) | ((uint32_t)to_storage(r1, kv_dtype) << 16);
-        uint32_t b = (uint32_t)to_storage(r2, kv_dtype) | ((uint32_t)to_storage(r3, kv_dtype) << 16);
-        if (!is_k && kv_dtype == YX_BF16 && (bf16_pair_is_wide(a) || bf16_pair_is_wide(b))) atomicOr(wide_v, 1u);
-        uint16_t *base = (uint16_t *)arena;
-        *(uint32_t *)(base + kv_off16(page, hkv, h, tok, 2 * lane)) = a;
-        *(uint32_t *)(base + kv_off16(page, hkv, h, tok, 64 + 2 * lane)) = b;
+#pragma unroll
+    for (int h = 0; h < HEADS; h++) {
+        const int head = head0 + h;
+        if (head >= heads) break;
+        const bool is_q = head < hq, is_k = !is_q && head < hq + hkv;
+        float r0 = lo[h].x, r1 = lo[h].y, r2 = hi[h].x, r3 = hi[h].y;
+        if (is_q || is_k) {
+            float ss = r0 * r0 + r1 * r1 + r2 * r2 + r3 * r3;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+            float r = 1.0f / sqrtf(ss / (float)D + eps);
+            const float *w = is_q ? q_norm : k_norm;
+            float2 wl = *(const float2 *)(w + 2 * lane), wh = *(const float2 *)(w + 64 + 2 * lane);
+            // Separate roundings (no fused multiply-add), as in the reference's Rust arithmetic.
+            float a0 = __fmul_rn(1.0f + wl.x, __fmul_rn(r0, r)), a1 = __fmul_rn(1.0f + wl.y, __fmul_rn(r1, r));
+            float b0 = __fmul_rn(1.0f + wh.x, __fmul_rn(r2, r)), b1 = __fmul_rn(1.0f + wh.y, __fmul_rn(r3, r));
+            r0 = __fsub_rn(__fmul_rn(a0, c0), __fmul_rn(b0, s0));
+            r2 = __fadd_rn(__fmul_rn(b0, c0), __fmul_rn(a0, s0));
+            r1 = __fsub_rn(__fmul_rn(a1, c1), __fmul_rn(b1, s1));
+            r3 = __fadd_rn(__fmul_rn(b1, c1), __fmul_rn(a1, s1));
+        }
+        if (is_q) {
+            float *q = q_out + ((size_t)row * hq + head) * D;
+            *(float2 *)(q + 2 * lane) = make_float2(r0, r1);
+            *(float2 *)(q + 64 + 2 * lane) = make_float2(r2, r3);
+            continue;
+        }
+        int kvh = is_k ? head - hq : head - hq - hkv;
+        char *arena = is_k ? k_arena : v_arena;
+        if (kv_dtype == YX_F32) {
+            float *d = (float *)arena + kv_off32(page, hkv, kvh, tok, 0);
+            *(float2 *)(d + 2 * lane) = make_float2(r0, r1);
+            *(float2 *)(d + 64 + 2 * lane) = make_float2(r2, r3);
+        } else {
+            uint32_t a = (uint32_t)to_storage(r0, kv_dtype) | ((uint32_t)to_storage(r1, kv_dtype) << 16);
+            uint32_t b = (uint32_t)to_storage(r2, kv_dtype) | ((uint32_t)to_storage(r3, kv_dtype) << 16);
+            if (!is_k && kv_dtype == YX_BF16 && (bf16_pair_is_wide(a) || bf16_pair_is_wide(b))) atomicOr(wide_v, 1u);
+            uint16_t *base = (uint16_t *)arena;
+            *(uint32_t *)(base + kv_off16(page, hkv, kvh, tok, 2 * lane)) = a;
+            *(uint32_t *)(base + kv_off16(page, hkv, kvh, tok, 64 + 2 * lane)) = b;
+        }
     }
 }
 
@@ -187,7 +206,8 @@ int launch_append(yx_ctx *ctx, yx_kv *kv, int layer, const void *k_rows, const v
     if (!ctx->smem_configured[4]) {
         // Keep the carve-out of the attention kernels these run between.
         cudaFuncSetAttribute(append_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-        cudaFuncSetAttribute(qk_rope_append_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        cudaFuncSetAttribute(qk_rope_append_kernel<1>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        cudaFuncSetAttribute(qk_rope_append_kernel<8>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         ctx->smem_configured[4] = true;
     }
     append_kernel<<<grid, 256, 0, ctx->stream>>>(k_rows, v_rows, src_dtype, ctx->d_slot, rows, kv->hkv, kv->dtype,
@@ -199,14 +219,19 @@ int launch_append(yx_ctx *ctx, yx_kv *kv, int layer, const void *k_rows, const v
 int launch_qk_rope_append(yx_ctx *ctx, yx_kv *kv, int layer, const float *qkv, const float *q_norm,
                           const float *k_norm, int hq, float eps, float *q_out) {
     uint32_t rows = ctx->pass.rows;
-    uint64_t warps = (uint64_t)rows * (hq + 2 * kv->hkv);
+    // Eight heads a warp once that gives every SM sixteen warps: 2048 rows of 48 heads took 42.6 us with a warp a head.
+    const int heads = hq + 2 * kv->hkv;
+    const bool several = (uint64_t)rows * ((heads + 7) / 8) >= 16u * (uint32_t)ctx->sm_count;
+    uint64_t warps = (uint64_t)rows * (several ? (heads + 7) / 8 : heads);
     uint32_t blocks = (uint32_t)((warps * 32 + 255) / 256);
     if (!ctx->smem_configured[4]) {
         cudaFuncSetAttribute(append_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-        cudaFuncSetAttribute(qk_rope_append_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        cudaFuncSetAttribute(qk_rope_append_kernel<1>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        cudaFuncSetAttribute(qk_rope_append_kernel<8>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         ctx->smem_configured[4] = true;
     }
-    qk_rope_append_kernel<<<blocks, 256, 0, ctx->stream>>>(qkv, q_norm, k_norm, ctx->d_pos, ctx->d_slot, rows, hq,
+    auto *kernel = several ? qk_rope_append_kernel<8> : qk_rope_append_kernel<1>;
+    kernel<<<blocks, 256, 0, ctx->stream>>>(qkv, q_norm, k_norm, ctx->d_pos, ctx->d_slot, rows, hq,
                                                           kv->hkv, eps, (const yx_rope *)kv->rope_dev + layer,
                                                           kv->dtype, kv->k(layer), kv->v(layer), q_out, kv->wide_v_dev);
     ctx->launches++;
