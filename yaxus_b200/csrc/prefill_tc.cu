@@ -6,16 +6,20 @@
 //
 // One CTA works on one item: up to 128 consecutive rows of one sequence (one M = 128 tile of
 // queries) for one query head, against that sequence's pages up to the last row's position.
-// Six warps:
-//   warps 0-3  softmax: thread t owns query row t and TMEM lane t.  It reads the scores of a
-//              128-key tile from TMEM, masks, keeps the running maximum and sum in f32,
-//              writes the probabilities back to TMEM as 16-bit pairs (over the scores), and
-//              rescales the output accumulator when the maximum has grown by more than 2^8
+// Ten warps:
+//   warps 0-7  softmax: two threads own a query row and its TMEM lane, a half of the row's 128 scores
+//              of a tile each.  They read them from TMEM, mask, agree on the maximum through shared
+//              memory, keep the running maximum and sum in f32, write the probabilities back to TMEM
+//              as 16-bit pairs (over the scores, which by then both halves hold in registers), and
+//              rescale the output accumulator when the maximum has grown by more than 2^8
 //              since the last rescale ("lazy" rescaling: until then the probabilities are
-//              simply allowed to exceed 1).
-//   warp 4     producer: page ids fetched 32 at a time, one 32 KiB bulk copy per K page and per
+//              simply allowed to exceed 1).  The softmax is what bounds this kernel (bf16 caches: two
+//              conversions, an exponential and half a dozen more instructions a score): with one thread
+//              a row and the cache's type looked up at run time, f32 queries of four 512-row chunks behind
+//              1024 keys on a bf16 cache (32 / 8 heads) took 225 us, now 131 us.
+//   warp 8     producer: page ids fetched 32 at a time, one 32 KiB bulk copy per K page and per
 //              V page (the cache layout is the 128-byte-swizzled operand layout already).
-//   warp 5     MMA issuer: S_j = Q K_j^T (M128 N128 K128, both operands K-major from shared
+//   warp 9     MMA issuer: S_j = Q K_j^T (M128 N128 K128, both operands K-major from shared
 //              memory) into one of two TMEM score buffers, then O += P_{j-1} V_{j-1} (P from
 //              TMEM, V MN-major from shared memory).  S_j is issued before P_{j-1}V_{j-1}, so
 //              the softmax of tile j-1 overlaps the tensor work of tile j.
@@ -36,13 +40,17 @@ constexpr int BN = 128;                  // keys per tile = one page
 constexpr int K_STAGES = 3, V_STAGES = 2;
 constexpr int PAGE_BYTES = PAGE * D * 2; // one (page, kv head) block of K or of V: 32 KiB
 constexpr int HALF_BYTES = PAGE * 128;   // one 64-dim half
-constexpr int SOFTMAX_WARPS = 4, PRODUCER_WARP = 4, MMA_WARP = 5;
-constexpr int THREADS = 6 * 32;
+constexpr int SOFTMAX_WARPS = 8, PRODUCER_WARP = 8, MMA_WARP = 9;
+constexpr int THREADS = 10 * 32;
 constexpr int TMEM_COLS = 512;
 constexpr int COL_S0 = 0, COL_S1 = 128, COL_O = 256;
 // barriers: q_full, k_full[3], k_empty[3], v_full[2], v_empty[2], s_full[2], p_full[2], pv_done
 constexpr int N_BARS = 1 + 2 * K_STAGES + 2 * V_STAGES + 2 + 2 + 1;
-constexpr int SMEM_BYTES = PAGE_BYTES * (2 + K_STAGES + V_STAGES) + N_BARS * 8 + 64;   // Q high, Q low, K ring, V ring
+// Q high, Q low, K ring, V ring, barriers, 64 bytes of odds and ends, what the halves of a row exchange.  (Nothing
+// static beside them: rounded up to the alignment of the operands it would not fit.)
+constexpr int SMEM_MISC = PAGE_BYTES * (2 + K_STAGES + V_STAGES) + N_BARS * 8;
+constexpr int SMEM_BYTES = SMEM_MISC + 64 + 2 * 2 * BM * 4;
+static_assert(SMEM_BYTES <= 227 * 1024, "shared memory of a CTA");
 
 struct TileParams {
     const void *q;
@@ -120,10 +128,12 @@ __device__ __forceinline__ float2 unpack_pair(uint32_t u, int bf16) {
     return __half22float2(*(__half2 *)&u);
 }
 
+template <bool BF16>
 __global__ void __launch_bounds__(THREADS, 1) prefill_tc_kernel(const TileParams P) {
     extern __shared__ __align__(1024) unsigned char smem[];
-    __shared__ uint32_t tmem_base_s;
-    __shared__ int abort_flag;
+    uint32_t &tmem_base_s = *(uint32_t *)(smem + SMEM_MISC);
+    int &abort_flag = *(int *)(smem + SMEM_MISC + 4);
+    auto row_part = (float (*)[2][BM])(smem + SMEM_MISC + 64);   // by parity of the tile: what the two halves of a row tell each other
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t s_q = smem_u32(smem);
     const uint32_t s_ql = s_q + PAGE_BYTES;
@@ -235,7 +245,7 @@ __global__ void __launch_bounds__(THREADS, 1) prefill_tc_kernel(const TileParams
     } else if (warp == MMA_WARP) {
         // ---- MMA issuer ----------------------------------------------------------------------
         if (lane == 0) {
-            const uint32_t idesc_qk = instr_desc(P.bf16, 0), idesc_pv = instr_desc(P.bf16, 1);
+            const uint32_t idesc_qk = instr_desc(BF16, 0), idesc_pv = instr_desc(BF16, 1);
             mbar_wait(b_q_full, 0, abortp, P.status, 33);
             tc_fence_after();
             uint32_t kph = 0, vph = 0;
@@ -250,7 +260,7 @@ __global__ void __launch_bounds__(THREADS, 1) prefill_tc_kernel(const TileParams
                 for (int k = 0; k < 8; k++) {   // 16 keys per step: two 8-row groups of the MN-major V tile
                     const uint64_t vdesc = smem_desc(v_base + k * 16 * 128, HALF_BYTES, 1024);
                     umma_ts(tmem + COL_O, tmem + (b ? COL_S1 : COL_S0) + k * 8, vdesc, idesc_pv, (j > 0 || k > 0) ? 1u : 0u);
-                    if (P.p_lo) umma_ts(tmem + COL_O, tmem + (b ? COL_S1 : COL_S0) + 64 + k * 8, vdesc, idesc_pv, 1u);
+                    if (BF16) umma_ts(tmem + COL_O, tmem + (b ? COL_S1 : COL_S0) + 64 + k * 8, vdesc, idesc_pv, 1u);
                 }
                 umma_commit(b_v_empty + 8 * vs);
                 umma_commit(b_pv_done);
@@ -276,34 +286,34 @@ __global__ void __launch_bounds__(THREADS, 1) prefill_tc_kernel(const TileParams
             if (n_tiles > 0 && !*abortp) issue_pv(n_tiles - 1);
         }
     } else {
-        // ---- softmax: thread t owns query row t -----------------------------------------------
-        const int r = threadIdx.x;
+        // ---- softmax: threads t and t + 128 own query row t, scores 64 half .. of a tile and dims 64 half .. of the output --
+        const int r = threadIdx.x & (BM - 1), half = warp >> 2;
         const bool valid = (uint32_t)r < it.n_rows;
         const uint32_t pos = it.pos0 + (valid ? r : 0);
         uint32_t klo = 0;
         if (P.window > 0 && pos + 1 > P.window) klo = pos + 1 - P.window;
         const uint32_t khi = pos;
-        const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);
+        const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
 
         // The query tile, converted to the cache's type, into the swizzled operand layout.
         {
             const size_t base = ((size_t)(it.row0 + (valid ? r : 0)) * P.hq + it.head) * D;
 #pragma unroll 4
-            for (int c = 0; c < 16; c++) {   // sixteen 16-byte chunks of the row
+            for (int c = 8 * half; c < 8 * half + 8; c++) {   // of the row's sixteen 16-byte chunks
                 float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
                 if (valid) {
                     a = load4_as_f32(P.q, P.q_dtype, base + c * 8);
                     b = load4_as_f32(P.q, P.q_dtype, base + c * 8 + 4);
                 }
-                const uint32_t w0 = pack_pair(a.x, a.y, P.bf16), w1 = pack_pair(a.z, a.w, P.bf16),
-                               w2 = pack_pair(b.x, b.y, P.bf16), w3 = pack_pair(b.z, b.w, P.bf16);
+                const uint32_t w0 = pack_pair(a.x, a.y, BF16), w1 = pack_pair(a.z, a.w, BF16),
+                               w2 = pack_pair(b.x, b.y, BF16), w3 = pack_pair(b.z, b.w, BF16);
                 const uint32_t addr = s_q + (c >> 3) * HALF_BYTES + r * 128 + (((c & 7) ^ (r & 7)) << 4);
                 asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(w0), "r"(w1), "r"(w2), "r"(w3) : "memory");
                 if (P.q_lo) {   // what the 16-bit rounding dropped
-                    const float2 h0 = unpack_pair(w0, P.bf16), h1 = unpack_pair(w1, P.bf16), h2 = unpack_pair(w2, P.bf16),
-                                 h3 = unpack_pair(w3, P.bf16);
-                    const uint32_t l0 = pack_pair(a.x - h0.x, a.y - h0.y, P.bf16), l1 = pack_pair(a.z - h1.x, a.w - h1.y, P.bf16),
-                                   l2 = pack_pair(b.x - h2.x, b.y - h2.y, P.bf16), l3 = pack_pair(b.z - h3.x, b.w - h3.y, P.bf16);
+                    const float2 h0 = unpack_pair(w0, BF16), h1 = unpack_pair(w1, BF16), h2 = unpack_pair(w2, BF16),
+                                 h3 = unpack_pair(w3, BF16);
+                    const uint32_t l0 = pack_pair(a.x - h0.x, a.y - h0.y, BF16), l1 = pack_pair(a.z - h1.x, a.w - h1.y, BF16),
+                                   l2 = pack_pair(b.x - h2.x, b.y - h2.y, BF16), l3 = pack_pair(b.z - h3.x, b.w - h3.y, BF16);
                     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr + PAGE_BYTES), "r"(l0), "r"(l1), "r"(l2), "r"(l3) : "memory");
                 }
             }
@@ -318,25 +328,27 @@ __global__ void __launch_bounds__(THREADS, 1) prefill_tc_kernel(const TileParams
             const uint32_t col_s = b ? COL_S1 : COL_S0;
             mbar_wait(b_s_full + 8 * b, (j >> 1) & 1u, abortp, P.status, 37);
             tc_fence_after();
-            uint32_t sr[4][32];
+            uint32_t sr[2][32];
 #pragma unroll
-            for (int c = 0; c < 4; c++) tmem_ld32(lane_addr + col_s + c * 32, sr[c]);
+            for (int c = 0; c < 2; c++) tmem_ld32(lane_addr + col_s + half * 64 + c * 32, sr[c]);
             tmem_ld_wait();
-            const uint32_t key0 = (it.page_begin + j) * PAGE;
-            const bool need_mask = key0 < klo || key0 + PAGE - 1 > khi;
-            float mx = -INFINITY;
+            const uint32_t key0 = (it.page_begin + j) * PAGE + half * 64;
+            if (key0 < klo || key0 + 63 > khi) {
 #pragma unroll
-            for (int c = 0; c < 4; c++)
+                for (int c = 0; c < 2; c++)
 #pragma unroll
-                for (int i = 0; i < 32; i++) {
-                    float s = __uint_as_float(sr[c][i]);
-                    if (need_mask) {
+                    for (int i = 0; i < 32; i++) {
                         const uint32_t key = key0 + c * 32 + i;
-                        if (key < klo || key > khi) s = -INFINITY;
+                        if (key < klo || key > khi) sr[c][i] = __float_as_uint(-INFINITY);
                     }
-                    sr[c][i] = __float_as_uint(s);
-                    mx = fmaxf(mx, s);
-                }
+            }
+            float mxs[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+            for (int i = 0; i < 64; i++) mxs[i & 3] = fmaxf(mxs[i & 3], __uint_as_float(sr[i >> 5][i & 31]));
+            float mx = fmaxf(fmaxf(mxs[0], mxs[1]), fmaxf(mxs[2], mxs[3]));
+            row_part[b][half][r] = mx;
+            asm volatile("bar.sync 1, %0;" ::"n"(SOFTMAX_WARPS * 32) : "memory");
+            mx = fmaxf(mx, row_part[b][half ^ 1][r]);
             // Lazy rescaling: keep the old reference maximum while the new one is within 2^8.
             float alpha = 1.f;
             bool rescale = false;
@@ -349,28 +361,25 @@ __global__ void __launch_bounds__(THREADS, 1) prefill_tc_kernel(const TileParams
             const float ms = (m_used == -INFINITY ? 0.f : m_used) * sl2;
             // Probabilities over the scores they came from: 128 keys as 64 packed columns, and
             // (bf16 caches) what the 8-bit mantissa dropped as 64 more.
-            float sum = 0.f;
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
+            float sums[4] = {0.f, 0.f, 0.f, 0.f};
+            {
                 uint32_t pr[32], pl[32];
 #pragma unroll
-                for (int c = 2 * h; c < 2 * h + 2; c++)
-#pragma unroll
-                    for (int i = 0; i < 32; i += 2) {
-                        const float p0 = fast_exp2(__uint_as_float(sr[c][i]) * sl2 - ms);
-                        const float p1 = fast_exp2(__uint_as_float(sr[c][i + 1]) * sl2 - ms);
-                        sum += p0 + p1;
-                        const uint32_t w = pack_pair(p0, p1, P.bf16);
-                        pr[(c & 1) * 16 + (i >> 1)] = w;
-                        if (P.p_lo) {
-                            const float2 hf = unpack_pair(w, P.bf16);
-                            pl[(c & 1) * 16 + (i >> 1)] = pack_pair(p0 - hf.x, p1 - hf.y, P.bf16);
-                        }
+                for (int i = 0; i < 64; i += 2) {
+                    const float p0 = fast_exp2(__uint_as_float(sr[i >> 5][i & 31]) * sl2 - ms);
+                    const float p1 = fast_exp2(__uint_as_float(sr[i >> 5][(i & 31) + 1]) * sl2 - ms);
+                    sums[(i >> 1) & 3] += p0 + p1;
+                    const uint32_t w = pack_pair(p0, p1, BF16);
+                    pr[i >> 1] = w;
+                    if (BF16) {
+                        const float2 hf = unpack_pair(w, BF16);
+                        pl[i >> 1] = pack_pair(p0 - hf.x, p1 - hf.y, BF16);
                     }
-                tmem_st32(lane_addr + col_s + h * 32, pr);
-                if (P.p_lo) tmem_st32(lane_addr + col_s + 64 + h * 32, pl);
+                }
+                tmem_st32(lane_addr + col_s + half * 32, pr);
+                if (BF16) tmem_st32(lane_addr + col_s + 64 + half * 32, pl);
             }
-            l += sum;
+            l += (sums[0] + sums[1]) + (sums[2] + sums[3]);
             tmem_st_wait();
             // The accumulator is quiet between P_{j-1}V_{j-1} and P_jV_j: rescale it here.
             if (j > 0) {
@@ -378,7 +387,7 @@ __global__ void __launch_bounds__(THREADS, 1) prefill_tc_kernel(const TileParams
                 tc_fence_after();
                 if (__any_sync(0xffffffffu, rescale)) {
 #pragma unroll 1
-                    for (int c = 0; c < 4; c++) {
+                    for (int c = 2 * half; c < 2 * half + 2; c++) {
                         uint32_t orow[32];
                         tmem_ld32(lane_addr + COL_O + c * 32, orow);
                         tmem_ld_wait();
@@ -396,10 +405,12 @@ __global__ void __launch_bounds__(THREADS, 1) prefill_tc_kernel(const TileParams
         if (n_tiles > 0) {
             mbar_wait(b_pv_done, (n_tiles - 1) & 1u, abortp, P.status, 39);
             tc_fence_after();
-            const float inv = 1.0f / l;
+            row_part[n_tiles & 1u][half][r] = l;   // (the parity whose maxima nobody reads any more)
+            asm volatile("bar.sync 1, %0;" ::"n"(SOFTMAX_WARPS * 32) : "memory");
+            const float inv = 1.0f / (row_part[n_tiles & 1u][0][r] + row_part[n_tiles & 1u][1][r]);
             const size_t obase = ((size_t)(it.row0 + (valid ? r : 0)) * P.hq + it.head) * D;
 #pragma unroll 1
-            for (int c = 0; c < 4; c++) {
+            for (int c = 2 * half; c < 2 * half + 2; c++) {
                 uint32_t orow[32];
                 tmem_ld32(lane_addr + COL_O + c * 32, orow);
                 tmem_ld_wait();
@@ -1022,9 +1033,10 @@ __global__ void __launch_bounds__(T2_THREADS_CONVERT, 1) prefill_tc2_bf16_kernel
 
 int launch_prefill_tc(yx_ctx *ctx, const TileArgs &a) {
     if (!ctx->smem_configured[6]) {
-        if (int rc = check_cuda(ctx, cudaFuncSetAttribute(prefill_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES),
-                                "prefill_tc: shared memory attribute"))
-            return rc;
+        for (auto *kernel : {prefill_tc_kernel<false>, prefill_tc_kernel<true>})
+            if (int rc = check_cuda(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES),
+                                    "prefill_tc: shared memory attribute"))
+                return rc;
         ctx->smem_configured[6] = true;
     }
     TileParams P{};
@@ -1072,7 +1084,8 @@ int launch_prefill_tc(yx_ctx *ctx, const TileArgs &a) {
         cudaError_t le = P.bf16 ? cudaLaunchKernelEx(&cfg, prefill_tc2_bf16_kernel, P) : cudaLaunchKernelEx(&cfg, prefill_tc2_f16_kernel, P);
         if (int rc = check_cuda(ctx, le, "prefill_tc2 kernel launch")) return rc;
     } else {
-        prefill_tc_kernel<<<a.n_items, THREADS, SMEM_BYTES, ctx->stream>>>(P);
+        if (P.bf16) prefill_tc_kernel<true><<<a.n_items, THREADS, SMEM_BYTES, ctx->stream>>>(P);
+        else prefill_tc_kernel<false><<<a.n_items, THREADS, SMEM_BYTES, ctx->stream>>>(P);
     }
     ctx->launches++;
     return check_cuda(ctx, cudaGetLastError(), "prefill_tc kernel");
