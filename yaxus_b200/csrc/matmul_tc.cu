@@ -718,6 +718,19 @@ int resident_pairs(yx_ctx *ctx, int *out) {
     return YX_OK;
 }
 
+// How many pairs share the k steps of `tiles` left-over tiles.  Either every tile is cut into the same number of
+// shares, which leaves some pairs idle, or all pairs take an equal share, which lets shares run over the end of a
+// tile: one more epilogue and one more share to add up for most pairs.  A k step takes 0.26 us and 2 ns a pass row
+// (62 GB/s into each SM, measured at 96 to 256 rows), the extra epilogue 3 us, adding up at all another 6; behind
+// whole rounds both are hidden.  A share of fewer than four k steps costs more to add up than it saves.
+uint32_t share_rest(uint32_t tiles, uint32_t ksteps, uint32_t pairs, uint32_t bt, bool hidden) {
+    const uint32_t most = std::max(1u, ksteps / 4), each = std::min(pairs / tiles, most);
+    const uint32_t all = std::min(pairs, tiles * most);
+    const float step = 0.26f + 0.002f * (float)bt, overrun = hidden ? 1.0f : each == 1 ? 9.0f : 3.0f;
+    const float even = step * (float)((ksteps + each - 1) / each), equal = step * (float)(tiles * ksteps) / (float)all;
+    return even <= equal + overrun ? tiles * each : all;
+}
+
 template <bool GLU>
 int matmul_pair_rows(yx_ctx *ctx, const float *x, const void *w, uint32_t T, uint32_t N, uint32_t K, float *out) {
     const size_t n = (size_t)T * K;
@@ -736,8 +749,7 @@ int matmul_pair_rows(yx_ctx *ctx, const float *x, const void *w, uint32_t T, uin
     a.pairs = (uint32_t)pairs;
     a.rounds = tiles / a.pairs;
     a.rest_units = (tiles - a.rounds * a.pairs) * a.ksteps;
-    // (a share of fewer than four k steps costs more to add up than it saves)
-    if (a.rest_units > 0) a.rest_pairs = std::min(a.pairs, std::max(1u, a.rest_units / std::min(4u, a.ksteps)));
+    if (a.rest_units > 0) a.rest_pairs = share_rest(tiles - a.rounds * a.pairs, a.ksteps, a.pairs, a.bt, a.rounds > 0);
     const uint32_t stage_bytes = W_BYTES + a.bt * 128u;
     a.stages = std::min<uint32_t>(TC_MAX_STAGES, (TC_SMEM_BUDGET - 1024) / stage_bytes);
     a.out = out;
