@@ -101,13 +101,18 @@ __global__ void qk_rope_append_kernel(const float *__restrict__ qkv, const float
     }
     const uint32_t slot = kv_slot[row], page = slot / PAGE;
     const int tok = (int)(slot % PAGE);
+    // (everything the rows need is asked for before the cosines keep the warp busy)
+    const float p = (float)pos[row], f0 = rope->inv_freq[2 * lane], f1 = rope->inv_freq[2 * lane + 1], conc = rope->concentration;
+    const float2 ql = *(const float2 *)(q_norm + 2 * lane), qh = *(const float2 *)(q_norm + 64 + 2 * lane);
+    const float2 kl = *(const float2 *)(k_norm + 2 * lane), kh = *(const float2 *)(k_norm + 64 + 2 * lane);
     float c0 = 0.f, s0 = 0.f, c1 = 0.f, s1 = 0.f;
     if (head0 < hq + hkv) {
-        float p = (float)pos[row];
-        float ang0 = __fmul_rn(p, rope->inv_freq[2 * lane]), ang1 = __fmul_rn(p, rope->inv_freq[2 * lane + 1]);
-        float conc = rope->concentration;
-        c0 = __fmul_rn((float)cos((double)ang0), conc), s0 = __fmul_rn((float)sin((double)ang0), conc);
-        c1 = __fmul_rn((float)cos((double)ang1), conc), s1 = __fmul_rn((float)sin((double)ang1), conc);
+        float ang0 = __fmul_rn(p, f0), ang1 = __fmul_rn(p, f1);
+        double sd0, cd0, sd1, cd1;
+        sincos((double)ang0, &sd0, &cd0);
+        sincos((double)ang1, &sd1, &cd1);
+        c0 = __fmul_rn((float)cd0, conc), s0 = __fmul_rn((float)sd0, conc);
+        c1 = __fmul_rn((float)cd1, conc), s1 = __fmul_rn((float)sd1, conc);
     }
 #pragma unroll
     for (int h = 0; h < HEADS; h++) {
@@ -120,8 +125,7 @@ __global__ void qk_rope_append_kernel(const float *__restrict__ qkv, const float
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
             float r = 1.0f / sqrtf(ss / (float)D + eps);
-            const float *w = is_q ? q_norm : k_norm;
-            float2 wl = *(const float2 *)(w + 2 * lane), wh = *(const float2 *)(w + 64 + 2 * lane);
+            const float2 wl = is_q ? ql : kl, wh = is_q ? qh : kh;
             // Separate roundings (no fused multiply-add), as in the reference's Rust arithmetic.
             float a0 = __fmul_rn(1.0f + wl.x, __fmul_rn(r0, r)), a1 = __fmul_rn(1.0f + wl.y, __fmul_rn(r1, r));
             float b0 = __fmul_rn(1.0f + wh.x, __fmul_rn(r2, r)), b1 = __fmul_rn(1.0f + wh.y, __fmul_rn(r3, r));
