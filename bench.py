@@ -485,10 +485,9 @@ def run_matmul(env, calls, warm, check=True):
         got = b.to_host(b.matmul_glu(x, sub))
         w_bits = sub.view(torch.int16).cpu().numpy().view(np.uint16)
         ref = o.swiglu(o.matmul(x.cpu().numpy(), w_bits, threads=host_cores()))
-        max_err = float(np.abs(got - ref).max())
+        full = b.to_host(b.matmul_glu(x, ws[0]))      # the same columns (the sums over k are cut elsewhere for another N)
+        max_err = max(float(np.abs(got - ref).max()), float(np.abs(full[:, rows] - ref).max()))
         assert max_err <= 2e-5 * max(1.0, float(np.abs(ref).max())), f"matmul_glu parity: {max_err}"
-        full = b.to_host(b.matmul_glu(x, ws[0]))      # and the full weight agrees with its slice
-        assert np.array_equal(full[:, rows], got), "matmul_glu: the full weight differs from its slice"
     env.barrier()
     out = torch.empty(T, N // 2, dtype=torch.float32, device=dev)
 
@@ -511,7 +510,7 @@ def run_matmul(env, calls, warm, check=True):
                             "frac": achieved / peaks["hbm"], "traffic": captured_traffic("matmul_rows_kernel_decode_matmul_glu")[0],
                             "traffic_source": captured_traffic("matmul_rows_kernel_decode_matmul_glu")[1], "peak_source": peaks["source"],
                             "kernel": "matmul_rows_kernel", "algorithmic_bytes": float(w_bytes),
-                            "how": "the whole call (packing, the matmul kernel, the finishing kernel) between two CUDA events"},
+                            "how": "the whole call (one kernel) between two CUDA events"},
                "host_us_per_call": host_us, "clocks": clocks, "gpu_launches": int(launches_per_call * calls),
                "parity_max_abs": max_err}
     del ws

@@ -30,9 +30,10 @@ def inputs(oracle, t, n, k):
     # few rows: each size of operand; one k step a CTA, a tile of 148 shares and more, several whole tiles a CTA
     (1, 1, 128), (7, 127, 256), (8, 129, 1024), (9, 300, 128), (16, 1000, 640), (17, 4100, 256), (32, 257, 1152),
     (1, 128, 19200), (3, 40000, 128), (32, 39000, 128),
-    (33, 1, 128), (64, 255, 128), (65, 257, 384), (256, 256, 1024), (257, 300, 640),   # fewer tiles than pairs
-    (40, 19300, 128), (300, 9700, 256),                                                # rounds and a remainder
-    (513, 6400, 128), (34, 18944, 128)])                                               # (the last: whole rounds where 74 pairs fit)
+    # many rows: fewer tiles than pairs; rounds and a remainder
+    (33, 1, 128), (64, 255, 128), (65, 257, 384), (280, 300, 512), (256, 256, 1024), (257, 300, 640),
+    (300, 9700, 256), (513, 6400, 128), (200, 18944, 128),
+    (40, 19300, 128), (49, 18000, 256), (128, 19201, 256), (97, 38400, 128)])
 def test_matmul_tiles(backend, oracle, t, n, k):
     x, w_bits = inputs(oracle, t, n, k)
     w, ref = backend.load_weight(w_bits), oracle.matmul(x, w_bits)
@@ -43,7 +44,9 @@ def test_matmul_tiles(backend, oracle, t, n, k):
     assert np.array_equal(backend.to_host(backend.matmul(xd, w)), first)
 
 
-@pytest.mark.parametrize("t,inner,k", [(1, 16, 128), (8, 1040, 256), (13, 48, 1024), (32, 9696, 128), (5, 24, 256), (33, 16, 128), (48, 144, 1024), (257, 1040, 256), (100, 24, 256), (35, 9696, 128)])
+@pytest.mark.parametrize("t,inner,k", [
+    (1, 16, 128), (8, 1040, 256), (13, 48, 1024), (32, 9696, 128), (5, 24, 256),
+    (33, 16, 128), (48, 144, 1024), (257, 1040, 256), (100, 24, 256), (150, 9696, 128), (35, 9696, 128), (60, 19456, 128)])
 def test_glu_tiles(backend, oracle, t, inner, k):
     x, w_bits = inputs(oracle, t, 2 * inner, k)
     w = backend.load_weight(w_bits)

@@ -44,6 +44,15 @@ constexpr int TC_THREADS = 10 * 32;
 constexpr int TC_TMA_WARP = 8, TC_MMA_WARP = 9;
 constexpr uint32_t W_BYTES = 128 * 128;     // a CTA's share of a stage's weights
 constexpr uint32_t TC_SMEM_BUDGET = 220 * 1024;
+// k steps summed in tensor memory before the epilogue takes them over into its own f32 sums: the tensor core drops what
+// lies below its accumulator's last place (see ROWS_CHAIN below).  Error of the result against 64-bit products, 512 rows
+// x [28672, 4096] with a GLU: one chain 1.9e-5, two library products 0.97e-5, chains of 16 0.64e-5; 80 rows 1.1e-5,
+// 0.96e-5, 0.57e-5; 80 rows x [50257, 4096] 8.5e-6, 2.7e-6, 3.3e-6.  Chains of 12 (2.9e-6 there) cost 80 rows another
+// 5 us of 69, chains of 8 another 8.  Where only two accumulators fit, a piece begins with a longer chain: it is what
+// the tensor cores have to do while the epilogue stores the piece before (2048 rows x [28672, 4096]: 608 us, with
+// chains of eight throughout 665, without chains 590).
+constexpr uint32_t TC_CHAIN = 16, TC_FIRST_CHAIN = 32;
+constexpr int TC_MAX_BUFS = 4;
 constexpr uint32_t GLU_GROUP = 16;          // gate and up rows alternate in a tile sixteen by sixteen: a warp holds both
 
 struct PairArgs {
@@ -54,6 +63,7 @@ struct PairArgs {
     uint32_t rounds;                  // whole rounds of tiles
     uint32_t rest_units, rest_pairs;  // k steps of the tiles after them, and the pairs that share those
     uint32_t stages;
+    uint32_t bufs, buf_columns;       // accumulators in tensor memory
     float *out;
     float *part;                      // [2 * rest_pairs shares][2 CTAs][bt][128]
     uint32_t *counters;               // [tiles left over][2 CTAs], zero between launches
@@ -95,6 +105,23 @@ struct Walk {
         p = Piece{round * a.pairs + pair, 0, a.ksteps, true};
         round++;
         return true;
+    }
+};
+
+// Where the chain of k steps that begins at k ends.
+__device__ __forceinline__ uint32_t chain_end(const PairArgs &a, const Piece &p, uint32_t k) {
+    uint32_t n = TC_CHAIN;
+    if (k == p.k0 && a.bufs == 2) n = min(TC_FIRST_CHAIN, max(TC_CHAIN, (p.k1 - p.k0) * 3 / 8));
+    return min(p.k1, k + n);
+}
+// Accumulators in turn, and the parity of the current round of them.
+struct AccTurn {
+    uint32_t buf = 0, round = 0;
+    __device__ __forceinline__ void next(uint32_t bufs) {
+        if (++buf == bufs) {
+            buf = 0;
+            round++;
+        }
     }
 };
 
@@ -140,7 +167,7 @@ template <bool GLU>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
 matmul_pair_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap x_map, const PairArgs a) {
     extern __shared__ __align__(1024) unsigned char smem[];
-    __shared__ __align__(8) uint64_t bar_store[2 * TC_MAX_STAGES + 4];
+    __shared__ __align__(8) uint64_t bar_store[2 * TC_MAX_STAGES + 2 * TC_MAX_BUFS];
     __shared__ uint32_t tmem_base_s;
     __shared__ int abort_flag;
     __shared__ int last_s;
@@ -149,7 +176,7 @@ matmul_pair_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_const
     const uint32_t S = a.stages, x_bytes = a.bt * 128u, stage_bytes = W_BYTES + x_bytes;   // x: bt / 2 rows, high and low part
     const uint32_t base = smem_u32(smem);
     const uint32_t b_full = smem_u32(bar_store), b_empty = b_full + 8 * TC_MAX_STAGES;
-    const uint32_t b_acc_full = b_empty + 8 * TC_MAX_STAGES, b_acc_empty = b_acc_full + 16;
+    const uint32_t b_acc_full = b_empty + 8 * TC_MAX_STAGES, b_acc_empty = b_acc_full + 8 * TC_MAX_BUFS;
     volatile int *abortp = &abort_flag;
 
     if (threadIdx.x == 0) {
@@ -158,7 +185,7 @@ matmul_pair_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_const
             mbar_init(b_full + 8 * s, 1);
             mbar_init(b_empty + 8 * s, 1);
         }
-        for (int b = 0; b < 2; b++) {
+        for (int b = 0; b < TC_MAX_BUFS; b++) {
             mbar_init(b_acc_full + 8 * b, 1);
             mbar_init(b_acc_empty + 8 * b, 16);   // a warp's arrival each, from both CTAs
         }
@@ -226,70 +253,92 @@ matmul_pair_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_const
         Walk walk(a, pair);
         Piece p;
         uint32_t s = 0, phase = 0;
-        for (uint32_t n = 0; walk.next(a, pair, p) && !*abortp; n++) {
-            const uint32_t buf = n & 1u, acc = tmem + buf * TC_MAX_BT;
-            if (n >= 2) mbar_wait(b_acc_empty + 8 * buf, ((n >> 1) - 1) & 1u, abortp, a.status, 502);
-            tc_fence_after();
-            for (uint32_t k = p.k0; k < p.k1; k++) {
-                mbar_wait(b_full + 8 * s, phase, abortp, a.status, 503);
-                if (*abortp) break;
+        AccTurn turn;
+        while (!*abortp && walk.next(a, pair, p)) {
+            for (uint32_t k0 = p.k0; k0 < p.k1 && !*abortp; turn.next(a.bufs)) {
+                const uint32_t acc = tmem + turn.buf * a.buf_columns, k_end = chain_end(a, p, k0);
+                if (turn.round > 0) mbar_wait(b_acc_empty + 8 * turn.buf, (turn.round - 1) & 1u, abortp, a.status, 502);
                 tc_fence_after();
-                const uint32_t w_lo = desc_lo(base + s * stage_bytes, 0), h_lo = w_lo + W_BYTES / 16, l_lo = h_lo + x_bytes / 32;
+                for (uint32_t k = k0; k < k_end; k++) {
+                    mbar_wait(b_full + 8 * s, phase, abortp, a.status, 503);
+                    if (*abortp) break;
+                    tc_fence_after();
+                    const uint32_t w_lo = desc_lo(base + s * stage_bytes, 0), h_lo = w_lo + W_BYTES / 16, l_lo = h_lo + x_bytes / 32;
 #pragma unroll
-                for (uint32_t kk = 0; kk < 4; kk++) umma2_ss_lo(acc, w_lo + 2 * kk, h_lo + 2 * kk, idesc, k > p.k0 || kk > 0);
+                    for (uint32_t kk = 0; kk < 4; kk++) umma2_ss_lo(acc, w_lo + 2 * kk, h_lo + 2 * kk, idesc, k > k0 || kk > 0);
 #pragma unroll
-                for (uint32_t kk = 0; kk < 4; kk++) umma2_ss_lo(acc, w_lo + 2 * kk, l_lo + 2 * kk, idesc, 1);
-                umma2_commit(b_empty + 8 * s);
-                if (++s == S) {
-                    s = 0;
-                    phase ^= 1u;
+                    for (uint32_t kk = 0; kk < 4; kk++) umma2_ss_lo(acc, w_lo + 2 * kk, l_lo + 2 * kk, idesc, 1);
+                    umma2_commit(b_empty + 8 * s);
+                    if (++s == S) {
+                        s = 0;
+                        phase ^= 1u;
+                    }
                 }
+                umma2_commit(b_acc_full + 8 * turn.buf);
+                k0 = k_end;
             }
-            umma2_commit(b_acc_full + 8 * buf);
         }
     } else if (warp < 8) {
         // ---- epilogue -------------------------------------------------------------------------
         Walk walk(a, pair);
         Piece p;
-        for (uint32_t n = 0; walk.next(a, pair, p); n++) {
-            const uint32_t buf = n & 1u, acc = tmem + buf * TC_MAX_BT + ((uint32_t)(warp & 3) << 21);
+        AccTurn turn;
+        while (walk.next(a, pair, p)) {
             const uint32_t wr = (warp & 3) * 32 + lane;   // weight row of this CTA's 128
             const uint32_t row = (p.tile / a.t_tiles) * TC_M + rank * 128u + wr, t0 = (p.tile % a.t_tiles) * a.bt;
-            mbar_wait(b_acc_full + 8 * buf, (n >> 1) & 1u, abortp, a.status, 504);
-            __syncwarp();   // (after a wait that ran out the warps go on, on whatever is there: their barriers below count all of them)
-            tc_fence_after();
             const uint32_t rest = p.whole ? 0u : p.tile - a.rounds * a.pairs;
-            // The pairs that share left-over tile `rest`.  Only the first of them may have begun in the tile before it,
-            // which makes this tile its second piece.
+            // The pairs that share left-over tile `rest`, found while it is being summed.  Only the first of them may
+            // have begun in the tile before it, which makes this tile its second piece.
             uint32_t q0 = 0, q1 = 0, second = 0;
             if (!p.whole) {
                 q0 = rest_owner(a, rest * a.ksteps);
                 q1 = rest_owner(a, (rest + 1) * a.ksteps - 1);
                 second = rest - rest_begin(a, q0) / a.ksteps;
             }
+            // This thread's sums: its weight row, 32 pass rows out of every 64.
+            constexpr int CHUNKS = TC_MAX_BT / 64;
+            const uint32_t c0 = 32u * (warp >> 2);
+            float sum[CHUNKS][32];
+#pragma unroll
+            for (int j = 0; j < CHUNKS; j++)
+#pragma unroll
+                for (int i = 0; i < 32; i++) sum[j][i] = 0.0f;
+            for (uint32_t k = p.k0; k < p.k1; k = chain_end(a, p, k), turn.next(a.bufs)) {
+                const uint32_t acc = tmem + turn.buf * a.buf_columns + ((uint32_t)(warp & 3) << 21);
+                mbar_wait(b_acc_full + 8 * turn.buf, turn.round & 1u, abortp, a.status, 504);
+                __syncwarp();   // (after a wait that ran out the warps go on, on whatever is there: their barriers below count all of them)
+                tc_fence_after();
+#pragma unroll
+                for (int j = 0; j < CHUNKS; j++) {
+                    if (c0 + 64 * j >= a.bt) break;
+#pragma unroll
+                    for (int h = 0; h < 32; h += 16) {   // (sixteen at a time: 32 more registers would spill)
+                        uint32_t r[16];
+                        tmem_ld16(acc + c0 + 64 * j + h, r);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int i = 0; i < 16; i++) sum[j][h + i] += __uint_as_float(r[i]);
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0)
+                    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(mapa(b_acc_empty + 8 * turn.buf, 0)) : "memory");
+            }
             // A share's sums: four pass rows of each of 128 weight rows, then the next four.
             auto share = [&](uint32_t q) { return (float4 *)(a.part + ((size_t)(2 * q + (q == q0 ? second : 0u)) * 2 + rank) * a.bt * 128u) + wr; };
-            for (uint32_t c = 32u * (warp >> 2); c < a.bt; c += 64) {
-                uint32_t r[32];
-                tmem_ld32(acc + c, r);
-                tmem_ld_wait();
-                if (p.whole) {
-                    float v[32];
 #pragma unroll
-                    for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
-                    store_rows<GLU>(a, v, t0 + c, row, lane);
+            for (int j = 0; j < CHUNKS; j++) {
+                const uint32_t c = c0 + 64 * j;
+                if (c >= a.bt) break;
+                if (p.whole) {
+                    store_rows<GLU>(a, sum[j], t0 + c, row, lane);
                 } else {
                     float4 *mine = share(pair) + c / 4 * 128u;
 #pragma unroll
-                    for (int i = 0; i < 8; i++)
-                        __stcg(mine + i * 128, make_float4(__uint_as_float(r[4 * i]), __uint_as_float(r[4 * i + 1]), __uint_as_float(r[4 * i + 2]),
-                                                           __uint_as_float(r[4 * i + 3])));
+                    for (int i = 0; i < 8; i++) __stcg(mine + i * 128, make_float4(sum[j][4 * i], sum[j][4 * i + 1], sum[j][4 * i + 2], sum[j][4 * i + 3]));
                 }
             }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0)
-                asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(mapa(b_acc_empty + 8 * buf, 0)) : "memory");
             if (p.whole) continue;
             // The last of the tile's shares to arrive adds all of them up, in the order of k.
             __threadfence();
@@ -390,6 +439,10 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float *__restrict
 constexpr int ROWS_THREADS = 14 * 32;
 constexpr int ROWS_CONVERT_WARP = 6, ROWS_CONVERTERS = 8;
 constexpr uint32_t ROWS_M = 128;
+// k steps summed in tensor memory before the epilogue takes them over into its own f32 sums.  The tensor core drops
+// what lies below its accumulator's last place: chains of 64 steps erred by 8.1e-6 of a GLU's result (16 rows x
+// [28672, 4096]), the mma.sync kernel by 4.2e-6.  Chains of 16 are at 4.0e-6.
+constexpr uint32_t ROWS_CHAIN = 16, ROWS_BUFS = 4;   // (and four accumulators: the tensor cores run on while an epilogue adds shares up)
 
 struct RowsArgs {
     const float *x;
@@ -427,16 +480,16 @@ template <int TP, bool GLU>
 __global__ void __launch_bounds__(ROWS_THREADS, 1)
 matmul_rows_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ RowsArgs a) {
     extern __shared__ __align__(1024) unsigned char smem[];
-    __shared__ __align__(8) uint64_t bar_store[2 * TC_MAX_STAGES + 4];
+    __shared__ __align__(8) uint64_t bar_store[2 * TC_MAX_STAGES + 2 * ROWS_BUFS];
     __shared__ uint32_t tmem_base_s;
     __shared__ int abort_flag;
     __shared__ int last_s;
     constexpr uint32_t NB = 2 * TP, X_BYTES = NB * 128, STAGE = W_BYTES + X_BYTES;
-    constexpr uint32_t TMEM = 2 * NB < 32 ? 32 : 2 * NB;   // two accumulators
+    constexpr uint32_t TMEM = ROWS_BUFS * NB;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t S = a.stages, base = smem_u32(smem);
     const uint32_t b_full = smem_u32(bar_store), b_empty = b_full + 8 * TC_MAX_STAGES;
-    const uint32_t b_acc_full = b_empty + 8 * TC_MAX_STAGES, b_acc_empty = b_acc_full + 16;
+    const uint32_t b_acc_full = b_empty + 8 * TC_MAX_STAGES, b_acc_empty = b_acc_full + 8 * ROWS_BUFS;
     volatile int *abortp = &abort_flag;
     const uint32_t u0 = share_begin(a, blockIdx.x), u1 = share_begin(a, blockIdx.x + 1);
 
@@ -460,7 +513,7 @@ matmul_rows_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_const
             mbar_init(b_full + 8 * s, 2);    // the weights' copy and the converting warp
             mbar_init(b_empty + 8 * s, 1);
         }
-        for (int b = 0; b < 2; b++) {
+        for (uint32_t b = 0; b < ROWS_BUFS; b++) {
             mbar_init(b_acc_full + 8 * b, 1);
             mbar_init(b_acc_empty + 8 * b, 4);
         }
@@ -498,11 +551,12 @@ matmul_rows_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_const
         // ---- MMA issuer -----------------------------------------------------------------------
         if (lane == 0) {
             constexpr uint32_t idesc = f16_instr_desc(true, false, ROWS_M, NB);
-            uint32_t s = 0, phase = 0, n = 0;
+            uint32_t s = 0, phase = 0, n = 0, piece_end = u0;
             for (uint32_t u = u0; u < u1 && !*abortp; n++) {
-                const uint32_t end = min(u1, (u / a.ksteps + 1) * a.ksteps);
-                const uint32_t buf = n & 1u, acc = tmem + buf * NB;
-                if (n >= 2) mbar_wait(b_acc_empty + 8 * buf, ((n >> 1) - 1) & 1u, abortp, a.status, 512);
+                if (u == piece_end) piece_end = min(u1, (u / a.ksteps + 1) * a.ksteps);
+                const uint32_t end = min(piece_end, u + ROWS_CHAIN);
+                const uint32_t buf = n % ROWS_BUFS, acc = tmem + buf * NB;
+                if (n >= ROWS_BUFS) mbar_wait(b_acc_empty + 8 * buf, (n / ROWS_BUFS - 1) & 1u, abortp, a.status, 512);
                 tc_fence_after();
                 for (uint32_t first = u; u < end; u++) {
                     mbar_wait(b_full + 8 * s, phase, abortp, a.status, 513);
@@ -565,47 +619,57 @@ matmul_rows_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_const
     } else {
         // ---- epilogue -------------------------------------------------------------------------
         uint32_t n = 0;
-        for (uint32_t u = u0; u < u1; n++) {
+        for (uint32_t u = u0; u < u1;) {
             const uint32_t tile = u / a.ksteps, end = min(u1, (tile + 1) * a.ksteps);
             const bool whole = end - u == a.ksteps;
-            const uint32_t buf = n & 1u, acc = tmem + buf * NB + ((uint32_t)warp << 21), wr = warp * 32 + lane, row = tile * ROWS_M + wr;
-            u = end;
-            mbar_wait(b_acc_full + 8 * buf, (n >> 1) & 1u, abortp, a.status, 515);
-            __syncwarp();   // (a wait that ran out does not stop these warps: their barriers below count all of them)
-            tc_fence_after();
+            const uint32_t wr = warp * 32 + lane, row = tile * ROWS_M + wr;
+            // The CTAs that share this tile, found while the tile is being summed (the divisions take a third of a
+            // microsecond).  Only the first of them may have begun in a tile before it: then this is its last piece.
+            uint32_t q0 = 0, q1 = 0, later = 0;
+            if (!whole) {
+                q0 = share_owner(a, tile * a.ksteps);
+                q1 = share_owner(a, (tile + 1) * a.ksteps - 1);
+                later = share_begin(a, q0) < tile * a.ksteps;
+            }
             float v[TP];
-            if constexpr (TP == 8) {
-                uint32_t r[16];
-                tmem_ld16(acc, r);
-                tmem_ld_wait();
 #pragma unroll
-                for (int i = 0; i < 8; i++) v[i] = __uint_as_float(r[i]) + __uint_as_float(r[8 + i]);
-            } else {
-#pragma unroll
-                for (int h = 0; h < TP / 16; h++) {
-                    uint32_t r[16], q[16];
-                    tmem_ld16(acc + 16 * h, r);
-                    tmem_ld16(acc + TP + 16 * h, q);
+            for (int i = 0; i < TP; i++) v[i] = 0.0f;
+            for (; u < end; n++) {
+                u = min(end, u + ROWS_CHAIN);
+                const uint32_t buf = n % ROWS_BUFS, acc = tmem + buf * NB + ((uint32_t)warp << 21);
+                mbar_wait(b_acc_full + 8 * buf, (n / ROWS_BUFS) & 1u, abortp, a.status, 515);
+                __syncwarp();   // (a wait that ran out does not stop these warps: their barriers below count all of them)
+                tc_fence_after();
+                if constexpr (TP == 8) {
+                    uint32_t r[16];
+                    tmem_ld16(acc, r);
                     tmem_ld_wait();
 #pragma unroll
-                    for (int i = 0; i < 16; i++) v[16 * h + i] = __uint_as_float(r[i]) + __uint_as_float(q[i]);
+                    for (int i = 0; i < 8; i++) v[i] += __uint_as_float(r[i]) + __uint_as_float(r[8 + i]);
+                } else {
+#pragma unroll
+                    for (int h = 0; h < TP / 16; h++) {
+                        uint32_t r[16], q[16];
+                        tmem_ld16(acc + 16 * h, r);
+                        tmem_ld16(acc + TP + 16 * h, q);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int i = 0; i < 16; i++) v[16 * h + i] += __uint_as_float(r[i]) + __uint_as_float(q[i]);
+                    }
                 }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(b_acc_empty + 8 * buf);
             }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(b_acc_empty + 8 * buf);
             if (whole) {
                 store_few<TP, GLU>(a, v, row, lane);
                 continue;
             }
-            auto share = [&](uint32_t q) {   // share of CTA q in this tile: its first piece or its last
-                return a.part + (size_t)(2 * q + (tile != share_begin(a, q) / a.ksteps)) * TP * 128u + wr;
-            };
+            auto share = [&](uint32_t q) { return a.part + (size_t)(2 * q + (q == q0 ? later : 0u)) * TP * 128u + wr; };
             float *mine = share(blockIdx.x);
 #pragma unroll
             for (int i = 0; i < TP; i++)
                 if (i < (int)a.T) __stcg(mine + i * 128, v[i]);
-            const uint32_t q0 = share_owner(a, tile * a.ksteps), q1 = share_owner(a, (tile + 1) * a.ksteps - 1);
             __threadfence();
             asm volatile("bar.sync 1, 128;" ::: "memory");
             if (threadIdx.x == 0) {
@@ -752,6 +816,8 @@ int matmul_pair_rows(yx_ctx *ctx, const float *x, const void *w, uint32_t T, uin
     if (a.rest_units > 0) a.rest_pairs = share_rest(tiles - a.rounds * a.pairs, a.ksteps, a.pairs, a.bt, a.rounds > 0);
     const uint32_t stage_bytes = W_BYTES + a.bt * 128u;
     a.stages = std::min<uint32_t>(TC_MAX_STAGES, (TC_SMEM_BUDGET - 1024) / stage_bytes);
+    a.bufs = a.bt <= 128 ? 4 : a.bt <= 160 ? 3 : 2;
+    a.buf_columns = 512 / a.bufs / 32 * 32;
     a.out = out;
     a.status = ctx->dev_status;
     if (int rc = ensure_buffer(ctx, (void **)&ctx->mm_part, &ctx->mm_part_cap,
