@@ -163,7 +163,9 @@ __device__ __forceinline__ void store_rows(const PairArgs &a, const float (&v)[3
     }
 }
 
-template <bool GLU>
+// CHUNKS: 64-row chunks of a tile, what an epilogue thread keeps in registers (two for up to
+// 128 pass rows: a step of 80 rows 391 us with room for four, 382 with two).
+template <bool GLU, int CHUNKS>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
 matmul_pair_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap x_map, const PairArgs a) {
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -296,7 +298,6 @@ matmul_pair_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_const
                 second = rest - rest_begin(a, q0) / a.ksteps;
             }
             // This thread's sums: its weight row, 32 pass rows out of every 64.
-            constexpr int CHUNKS = TC_MAX_BT / 64;
             const uint32_t c0 = 32u * (warp >> 2);
             float sum[CHUNKS][32];
 #pragma unroll
@@ -756,11 +757,11 @@ int ensure_counters(yx_ctx *ctx, size_t n) {
 }
 
 // CTA pairs that are on the chip together (a GPC with an odd number of SMs leaves one out).
-template <bool GLU>
+template <bool GLU, int CHUNKS>
 int resident_pairs(yx_ctx *ctx, int *out) {
-    int &n = ctx->mm_pairs[GLU];
+    int &n = ctx->mm_pairs[GLU][CHUNKS == 4];
     if (n == 0) {
-        auto *kernel = matmul_pair_kernel<GLU>;
+        auto *kernel = matmul_pair_kernel<GLU, CHUNKS>;
         if (int rc = check_cuda(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_BUDGET),
                                 "matmul: shared memory attribute"))
             return rc;
@@ -795,12 +796,12 @@ uint32_t share_rest(uint32_t tiles, uint32_t ksteps, uint32_t pairs, uint32_t bt
     return even <= equal + overrun ? tiles * each : all;
 }
 
-template <bool GLU>
+template <bool GLU, int CHUNKS>
 int matmul_pair_rows(yx_ctx *ctx, const float *x, const void *w, uint32_t T, uint32_t N, uint32_t K, float *out) {
     const size_t n = (size_t)T * K;
     if (int rc = ensure_buffer(ctx, (void **)&ctx->mm_packed, &ctx->mm_packed_cap, n * 4)) return rc;
     int pairs = 0;
-    if (int rc = resident_pairs<GLU>(ctx, &pairs)) return rc;
+    if (int rc = resident_pairs<GLU, CHUNKS>(ctx, &pairs)) return rc;
 
     PairArgs a{};
     a.T = T;
@@ -841,7 +842,7 @@ int matmul_pair_rows(yx_ctx *ctx, const float *x, const void *w, uint32_t T, uin
                                   dim3((unsigned)((n / 8 + 255) / 256)), dim3(256), 0, x, n, hi, lo))
         return rc;
     const uint32_t grid = 2 * (a.rounds > 0 ? a.pairs : a.rest_pairs);
-    return launch_dependent(ctx, "matmul kernel launch", matmul_pair_kernel<GLU>, dim3(grid), dim3(TC_THREADS), a.stages * stage_bytes, w_map, x_map, a);
+    return launch_dependent(ctx, "matmul kernel launch", matmul_pair_kernel<GLU, CHUNKS>, dim3(grid), dim3(TC_THREADS), a.stages * stage_bytes, w_map, x_map, a);
 }
 
 template <int TP, bool GLU>
@@ -883,7 +884,7 @@ int matmul_tc(yx_ctx *ctx, const float *x, const void *w, uint32_t T, uint32_t N
     if (T <= 8) return matmul_few_rows<8, GLU>(ctx, x, w, T, N, K, out);
     if (T <= 16) return matmul_few_rows<16, GLU>(ctx, x, w, T, N, K, out);
     if (T <= 32) return matmul_few_rows<32, GLU>(ctx, x, w, T, N, K, out);
-    return matmul_pair_rows<GLU>(ctx, x, w, T, N, K, out);
+    return T <= 128 ? matmul_pair_rows<GLU, 2>(ctx, x, w, T, N, K, out) : matmul_pair_rows<GLU, 4>(ctx, x, w, T, N, K, out);
 }
 
 }  // namespace
