@@ -17,14 +17,14 @@
 // up in order.  The shares come first in a pair's work, so that the adding up hides under whole tiles.  Adding up
 // is a chain of L2 latencies: with one warp to a lane quarter and one share at a time it took 15 to 20 us.
 //
-// Large passes are bound by the tensor cores: 2048 rows on 4096 -> 28672 (gate and up) take 625 us, 1.54 PFLOP/s
+// Large passes are bound by the tensor cores: 2048 rows on 4096 -> 28672 (gate and up) take 608 us, 1.58 PFLOP/s
 // of bf16 products; 80 rows by the weights' way through L2 and shared memory: 412 MB in 100 us.  Against two
 // library products (high part, then low part added to it) and a SwiGLU kernel, whole steps of one layer went from
-// 2151 to 1776 us (2048 rows) and from 1244 to 387 us (80 rows).
+// 2151 to 1700 us (2048 rows) and from 1244 to 382 us (80 rows).
 //
 // Warps 0-7 epilogue (two to each 32 lanes of tensor memory, taking turns at 32 pass rows), warp 8 TMA, warp 9
-// issues the MMAs (first CTA of the pair).  All waits are bounded; on expiry the CTA records where, stops waiting anywhere, frees its
-// tensor memory together with its partner and returns.
+// issues the MMAs (first CTA of the pair).  All waits are bounded; on expiry the CTA records where, stops waiting
+// anywhere, frees its tensor memory together with its partner and returns.
 #include <cuda.h>
 
 #include <algorithm>
@@ -164,7 +164,7 @@ __device__ __forceinline__ void store_rows(const PairArgs &a, const float (&v)[3
 }
 
 // CHUNKS: 64-row chunks of a tile, what an epilogue thread keeps in registers (two for up to
-// 128 pass rows: a step of 80 rows 391 us with room for four, 382 with two).
+// 128 pass rows, three for up to 192: steps of 80 and of 311 rows take 391 and 453 us with room for four, 382 and 437 so).
 template <bool GLU, int CHUNKS>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
 matmul_pair_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap x_map, const PairArgs a) {
@@ -436,7 +436,7 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float *__restrict
 // Bound by HBM from some 200 MB on (one row on 28672 x 4096: 45 us, the part above a launch's fixed 8 to 12 us at
 // 7.2 TB/s), by a chain of latencies below.  The kernel with weights straight from global memory into mma.sync
 // fragments, a packing kernel before it and a finishing kernel behind took 58 us for sixteen rows of that weight;
-// steps went from 419 to 374 us (one row, large), 538 to 440 us (sixteen rows), 417 to 340 us (one row, small).
+// steps went from 419 to 352 us (one row, large), 538 to 424 us (sixteen rows), 417 to 340 us (one row, small).
 constexpr int ROWS_THREADS = 14 * 32;
 constexpr int ROWS_CONVERT_WARP = 6, ROWS_CONVERTERS = 8;
 constexpr uint32_t ROWS_M = 128;
@@ -759,7 +759,7 @@ int ensure_counters(yx_ctx *ctx, size_t n) {
 // CTA pairs that are on the chip together (a GPC with an odd number of SMs leaves one out).
 template <bool GLU, int CHUNKS>
 int resident_pairs(yx_ctx *ctx, int *out) {
-    int &n = ctx->mm_pairs[GLU][CHUNKS == 4];
+    int &n = ctx->mm_pairs[GLU][CHUNKS - 2];
     if (n == 0) {
         auto *kernel = matmul_pair_kernel<GLU, CHUNKS>;
         if (int rc = check_cuda(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_BUDGET),
@@ -781,6 +781,12 @@ int resident_pairs(yx_ctx *ctx, int *out) {
     }
     *out = n;
     return YX_OK;
+}
+
+// Pass rows are spread evenly over as few tiles as hold them: 300 rows are two tiles of 160, not 256 and 64.
+uint32_t tile_rows(uint32_t T) {
+    const uint32_t tiles = (T + TC_MAX_BT - 1) / TC_MAX_BT;
+    return ((T + tiles - 1) / tiles + 31) / 32 * 32;
 }
 
 // How many pairs share the k steps of `tiles` left-over tiles.  Either every tile is cut into the same number of
@@ -806,9 +812,8 @@ int matmul_pair_rows(yx_ctx *ctx, const float *x, const void *w, uint32_t T, uin
     PairArgs a{};
     a.T = T;
     a.cols = GLU ? N / 2 : N;
-    // Pass rows are spread evenly over as few tiles as hold them: 300 rows are two tiles of 160, not 256 and 64.
     a.t_tiles = (T + TC_MAX_BT - 1) / TC_MAX_BT;
-    a.bt = ((T + a.t_tiles - 1) / a.t_tiles + 31) / 32 * 32;
+    a.bt = tile_rows(T);
     a.ksteps = K / TC_KSTEP;
     const uint32_t tiles = ((N + TC_M - 1) / TC_M) * a.t_tiles;
     a.pairs = (uint32_t)pairs;
@@ -884,7 +889,10 @@ int matmul_tc(yx_ctx *ctx, const float *x, const void *w, uint32_t T, uint32_t N
     if (T <= 8) return matmul_few_rows<8, GLU>(ctx, x, w, T, N, K, out);
     if (T <= 16) return matmul_few_rows<16, GLU>(ctx, x, w, T, N, K, out);
     if (T <= 32) return matmul_few_rows<32, GLU>(ctx, x, w, T, N, K, out);
-    return T <= 128 ? matmul_pair_rows<GLU, 2>(ctx, x, w, T, N, K, out) : matmul_pair_rows<GLU, 4>(ctx, x, w, T, N, K, out);
+    const uint32_t rows = tile_rows(T);
+    if (rows <= 128) return matmul_pair_rows<GLU, 2>(ctx, x, w, T, N, K, out);
+    if (rows <= 192) return matmul_pair_rows<GLU, 3>(ctx, x, w, T, N, K, out);
+    return matmul_pair_rows<GLU, 4>(ctx, x, w, T, N, K, out);
 }
 
 }  // namespace

@@ -347,7 +347,7 @@ struct yx_ctx {
     uint32_t *mm_counters = nullptr;       // arrivals at the matmul tiles several CTAs share; zero between launches
     size_t mm_counters_cap = 0;
     bool mm_rows_configured[2][3] = {};    // opt-in to large shared memory of the few-row matmul kernels
-    int mm_pairs[2][2] = {};               // CTA pairs of the matmul kernel (plain or GLU, small or large tiles) that fit the chip together
+    int mm_pairs[2][3] = {};               // CTA pairs of the matmul kernel (plain or GLU, by the tile's size) that fit the chip together
     uint32_t *idx_dev = nullptr;           // token ids / row indices / argmax parts of the model operators
     size_t idx_cap = 0;
     uint32_t *pick_counters = nullptr;     // argmax: arrivals per row, zero between launches
