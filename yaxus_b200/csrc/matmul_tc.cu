@@ -20,7 +20,7 @@
 // Large passes are bound by the tensor cores: 2048 rows on 4096 -> 28672 (gate and up) take 608 us, 1.58 PFLOP/s
 // of bf16 products; 80 rows by the weights' way through L2 and shared memory: 412 MB in 100 us.  Against two
 // library products (high part, then low part added to it) and a SwiGLU kernel, whole steps of one layer went from
-// 2151 to 1700 us (2048 rows) and from 1244 to 382 us (80 rows).
+// 2151 to 1700 us (2048 rows) and from 1244 to 399 us (80 rows).
 //
 // Warps 0-7 epilogue (two to each 32 lanes of tensor memory, taking turns at 32 pass rows), warp 8 TMA, warp 9
 // issues the MMAs (first CTA of the pair).  All waits are bounded; on expiry the CTA records where, stops waiting
@@ -46,11 +46,12 @@ constexpr uint32_t W_BYTES = 128 * 128;     // a CTA's share of a stage's weight
 constexpr uint32_t TC_SMEM_BUDGET = 220 * 1024;
 // k steps summed in tensor memory before the epilogue takes them over into its own f32 sums: the tensor core drops what
 // lies below its accumulator's last place (see ROWS_CHAIN below).  Error of the result against 64-bit products, 512 rows
-// x [28672, 4096] with a GLU: one chain 1.9e-5, two library products 0.97e-5, chains of 16 0.64e-5; 80 rows 1.1e-5,
-// 0.96e-5, 0.57e-5; 80 rows x [50257, 4096] 8.5e-6, 2.7e-6, 3.3e-6.  Chains of 12 (2.9e-6 there) cost 80 rows another
-// 5 us of 69, chains of 8 another 8.  Where only two accumulators fit, a piece begins with a longer chain: it is what
-// the tensor cores have to do while the epilogue stores the piece before (2048 rows x [28672, 4096]: 608 us, with
-// chains of eight throughout 665, without chains 590).
+// x [28672, 4096] with a GLU: one chain 1.9e-5, two library products 0.97e-5, chains of 16 0.64e-5.  Tiles of up to 128
+// rows take chains of eight, without which 80 rows x [50257, 4096] lose against the library (8.5e-6 in one chain, 3.3e-6
+// in chains of 16, 2.7e-6 in chains of eight and in the library); a step of 80 rows pays 19 us of 399 for that.  Where
+// only two accumulators fit, a piece begins with a longer chain: it is what the tensor cores have to do while the
+// epilogue stores the piece before (2048 rows x [28672, 4096]: 608 us, with chains of eight throughout 665, without
+// chains 590).
 constexpr uint32_t TC_CHAIN = 16, TC_FIRST_CHAIN = 32;
 constexpr int TC_MAX_BUFS = 4;
 constexpr uint32_t GLU_GROUP = 16;          // gate and up rows alternate in a tile sixteen by sixteen: a warp holds both
@@ -110,7 +111,7 @@ struct Walk {
 
 // Where the chain of k steps that begins at k ends.
 __device__ __forceinline__ uint32_t chain_end(const PairArgs &a, const Piece &p, uint32_t k) {
-    uint32_t n = TC_CHAIN;
+    uint32_t n = a.bufs == TC_MAX_BUFS ? TC_CHAIN / 2 : TC_CHAIN;
     if (k == p.k0 && a.bufs == 2) n = min(TC_FIRST_CHAIN, max(TC_CHAIN, (p.k1 - p.k0) * 3 / 8));
     return min(p.k1, k + n);
 }
