@@ -437,14 +437,15 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float *__restrict
 // Bound by HBM from some 200 MB on (one row on 28672 x 4096: 45 us, the part above a launch's fixed 8 to 12 us at
 // 7.2 TB/s), by a chain of latencies below.  The kernel with weights straight from global memory into mma.sync
 // fragments, a packing kernel before it and a finishing kernel behind took 58 us for sixteen rows of that weight;
-// steps went from 419 to 352 us (one row, large), 538 to 424 us (sixteen rows), 417 to 340 us (one row, small).
+// steps went from 419 to 360 us (one row, large), 538 to 424 us (sixteen rows), 417 to 340 us (one row, small).
 constexpr int ROWS_THREADS = 14 * 32;
 constexpr int ROWS_CONVERT_WARP = 6, ROWS_CONVERTERS = 8;
 constexpr uint32_t ROWS_M = 128;
 // k steps summed in tensor memory before the epilogue takes them over into its own f32 sums.  The tensor core drops
 // what lies below its accumulator's last place: chains of 64 steps erred by 8.1e-6 of a GLU's result (16 rows x
-// [28672, 4096]), the mma.sync kernel by 4.2e-6.  Chains of 16 are at 4.0e-6.
-constexpr uint32_t ROWS_CHAIN = 16, ROWS_BUFS = 4;   // (and four accumulators: the tensor cores run on while an epilogue adds shares up)
+// [28672, 4096]), the mma.sync kernel by 4.2e-6.  Chains of 16 are
+// at 4.0e-6 (but 3.9e-6 against 3.7e-6 for twenty rows x [11264, 2048]), chains of eight at 3.7e-6 for 1.5 % of a step.
+constexpr uint32_t ROWS_CHAIN = 8, ROWS_BUFS = 4;   // (and four accumulators: the tensor cores run on while an epilogue adds shares up)
 
 struct RowsArgs {
     const float *x;
