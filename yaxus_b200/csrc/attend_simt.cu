@@ -83,7 +83,7 @@ __device__ __forceinline__ void merge_parts(const RowMerge &fin, const Merge &mg
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) cm = fmaxf(cm, __shfl_xor_sync(0xffffffffu, cm, off));
         const float nm = fmaxf(mx, cm), r = __expf(mx - nm), w = live ? __expf(ml.x - nm) : 0.0f;
-        float ls = live ? ml.y * w : 0.0f;
+        float ls = ml.y * w;   // (a sum that is no number has weight 0 and stays no number: the row shows it)
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) ls += __shfl_xor_sync(0xffffffffu, ls, off);
         l = l * r + ls;
