@@ -70,3 +70,29 @@ def test_unaligned_rows(backend, oracle, t):
     xd.copy_(torch.from_numpy(x))
     got = backend.to_host(backend.matmul(xd, backend.load_weight(w_bits)))
     assert (np.abs(got - oracle.matmul(x, w_bits)) <= TOL * magnitudes(x, w_bits)).all()
+
+
+def test_no_scratch_grows_where_fewer_rows_follow_more():
+    # Calls recorded into a graph after passes of as many rows: growing a buffer would
+    # synchronise the stream, which ends the recording.
+    from yaxus_b200 import CudaBackend
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        b = CudaBackend(0, stream=stream)
+        x = torch.randn(512, 256, device=b.device)
+        few, many, odd = (torch.randn(n, 256, device=b.device).bfloat16() for n in (256, 9000, 2 * 24))
+        for rows in (1, 512):
+            b.matmul(x[:rows], few)
+        b.matmul(x[:1], many)
+        b.matmul_glu(x[:1], odd)
+        b.sync()
+        calls = [(b.matmul, 16, many), (b.matmul, 300, many), (b.matmul, 100, many), (b.matmul_glu, 16, odd)]
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            outs = [op(x[:rows], w) for op, rows, w in calls]
+        graph.replay()
+        b.sync()
+        for out, (op, rows, w) in zip(outs, calls):
+            assert torch.equal(out, op(x[:rows], w))
+    del graph
+    b.close()

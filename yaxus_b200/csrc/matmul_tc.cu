@@ -441,6 +441,7 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float *__restrict
 constexpr int ROWS_THREADS = 14 * 32;
 constexpr int ROWS_CONVERT_WARP = 6, ROWS_CONVERTERS = 8;
 constexpr uint32_t ROWS_M = 128;
+constexpr uint32_t ROWS_MAX = 32;           // pass rows
 // k steps summed in tensor memory before the epilogue takes them over into its own f32 sums.  The tensor core drops
 // what lies below its accumulator's last place: chains of 64 steps erred by 8.1e-6 of a GLU's result (16 rows x
 // [28672, 4096]), the mma.sync kernel by 4.2e-6.  Chains of 16 are
@@ -828,11 +829,11 @@ int matmul_pair_rows(yx_ctx *ctx, const float *x, const void *w, uint32_t T, uin
     a.buf_columns = 512 / a.bufs / 32 * 32;
     a.out = out;
     a.status = ctx->dev_status;
-    if (int rc = ensure_buffer(ctx, (void **)&ctx->mm_part, &ctx->mm_part_cap,
-                               std::max<size_t>((size_t)a.rest_pairs * 2 * 2 * a.bt * 128 * sizeof(float), 16)))
-        return rc;
+    // The most any pass needs (39 MB), so that a call that is being recorded into a graph finds it whatever passes came
+    // before: the shares' room does not grow with the rows (512 rows may leave no tile over, 100 rows many).
+    if (int rc = ensure_buffer(ctx, (void **)&ctx->mm_part, &ctx->mm_part_cap, (size_t)a.pairs * 2 * 2 * TC_MAX_BT * 128 * sizeof(float))) return rc;
     a.part = ctx->mm_part;
-    if (int rc = ensure_counters(ctx, 2 * (tiles - a.rounds * a.pairs))) return rc;
+    if (int rc = ensure_counters(ctx, 2 * a.pairs)) return rc;
     a.counters = ctx->mm_counters;
 
     CUtensorMap w_map, x_map;
@@ -876,7 +877,8 @@ int matmul_few_rows(yx_ctx *ctx, const float *x, const void *w, uint32_t T, uint
     a.x_vec16 = ((uintptr_t)x & 15u) == 0;
     a.out = out;
     a.status = ctx->dev_status;
-    if (int rc = ensure_buffer(ctx, (void **)&ctx->mm_part, &ctx->mm_part_cap, (size_t)2 * a.ctas * TP * 128 * sizeof(float))) return rc;
+    // (for any number of rows and any weight, as in matmul_pair_rows: one row may be followed by sixteen in a recording)
+    if (int rc = ensure_buffer(ctx, (void **)&ctx->mm_part, &ctx->mm_part_cap, (size_t)2 * ctx->sm_count * ROWS_MAX * 128 * sizeof(float))) return rc;
     if (int rc = ensure_counters(ctx, tiles)) return rc;
     a.part = ctx->mm_part;
     a.counters = ctx->mm_counters;

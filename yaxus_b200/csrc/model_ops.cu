@@ -323,7 +323,8 @@ int matmul_impl(yx_ctx *ctx, const float *x, const void *w_bf16, uint32_t T, uin
     if (tensor && (!glu || cols % 16 == 0)) return launch_matmul_tc(ctx, x, w, T, N, K, glu != 0, out);
     float *dst = out;
     if (glu) {
-        if (int rc = ensure_buffer(ctx, (void **)&ctx->mm_sums, &ctx->mm_sums_cap, (size_t)T * N * sizeof(float))) return rc;
+        // (room for 32 rows at least: see matmul_few_rows)
+        if (int rc = ensure_buffer(ctx, (void **)&ctx->mm_sums, &ctx->mm_sums_cap, (size_t)std::max(T, 32u) * N * sizeof(float))) return rc;
         dst = ctx->mm_sums;
     }
     if (tensor) {
