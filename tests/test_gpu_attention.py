@@ -348,3 +348,14 @@ def test_empty_pass(backend):
     backend.sync()
     assert out.shape == (0, 1024)
     kv.close()
+
+
+def test_lse_combine_of_strided_parts(backend):
+    # transposed triples: what the call copies must live until it has been queued
+    gen = torch.Generator(device=backend.device)
+    gen.manual_seed(3)
+    m, l = (torch.rand(300, 7, generator=gen, device=backend.device) for _ in range(2))
+    o = torch.randn(300, 7, 128, generator=gen, device=backend.device)
+    got = backend.lse_combine(m.T, l.T, o.transpose(0, 1))
+    want = backend.lse_combine(m.T.contiguous(), l.T.contiguous(), o.transpose(0, 1).contiguous())
+    assert torch.equal(got, want)

@@ -342,9 +342,9 @@ class CudaBackend:
                     out_dtype: torch.dtype = torch.float32) -> torch.Tensor:
         """m, l `[parts, n]`, o `[parts, n, 128]` -> `[n, 128]`."""
         parts, n = m.shape[0], m[0].numel()
+        m, l, o = m.contiguous(), l.contiguous(), o.contiguous()   # (named: alive until the launch is queued)
         out = torch.empty(n, HEAD_DIM, dtype=out_dtype, device=self.device)
-        self._L.yx_lse_combine(self._ctx, parts, _ptr(m.contiguous()), _ptr(l.contiguous()), _ptr(o.contiguous()), n,
-                               _ptr(out), _YX_DTYPE[out_dtype])
+        self._L.yx_lse_combine(self._ctx, parts, _ptr(m), _ptr(l), _ptr(o), n, _ptr(out), _YX_DTYPE[out_dtype])
         return out
 
     # ---- keys split across GPUs --------------------------------------------------------
