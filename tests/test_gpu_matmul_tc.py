@@ -72,6 +72,18 @@ def test_unaligned_rows(backend, oracle, t):
     assert (np.abs(got - oracle.matmul(x, w_bits)) <= TOL * magnitudes(x, w_bits)).all()
 
 
+def test_more_outputs_than_a_32_bit_thread_index_reaches(backend):
+    # a warp an output: 2^27 outputs are 2^32 threads
+    t, n = 4097, 32768
+    gen = torch.Generator(device=backend.device)
+    gen.manual_seed(11)
+    x, w = torch.randn(t, 1, generator=gen, device=backend.device), backend.load_weight(torch.randn(n, 1, generator=gen, device=backend.device))
+    torch.full((t, n), float("nan"), device=backend.device)               # (given back at once: the result's memory, most likely)
+    got = backend.matmul(x, w)
+    backend.sync()
+    assert torch.equal(got, x * w.float().T)                              # one product each: the same rounding
+
+
 def test_no_scratch_grows_where_fewer_rows_follow_more():
     # Calls recorded into a graph after passes of as many rows: growing a buffer would
     # synchronise the stream, which ends the recording.

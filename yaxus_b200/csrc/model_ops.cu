@@ -17,17 +17,17 @@ namespace {
 
 using namespace dev;
 
-// Any shape the tensor-core kernel does not take (K not a multiple of 128): a warp per output.
-__global__ void matmul_any_kernel(const float *__restrict__ x, const __nv_bfloat16 *__restrict__ w, uint32_t T, uint32_t N,
-                                  uint32_t K, float *__restrict__ out) {
-    const uint32_t o = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (o >= T * N) return;
-    const uint32_t t = o / N, n = o - t * N;
+// Any shape the tensor-core kernel does not take (K not a multiple of 128): a warp per output, pass rows in the grid's y
+// extent (a thread's number among all outputs' does not fit in 32 bits from 2^27 outputs on).
+__global__ void matmul_any_kernel(const float *__restrict__ x, const __nv_bfloat16 *__restrict__ w, uint32_t N, uint32_t K,
+                                  float *__restrict__ out) {
+    const uint32_t n = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), t = blockIdx.y, lane = threadIdx.x & 31;
+    if (n >= N) return;
     float s = 0.0f;
     for (uint32_t k = lane; k < K; k += 32) s += __bfloat162float(w[(size_t)n * K + k]) * x[(size_t)t * K + k];
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
-    if (lane == 0) out[o] = s;
+    if (lane == 0) out[(size_t)t * N + n] = s;
 }
 
 __global__ void swiglu_kernel(const float *__restrict__ x, uint32_t rows, uint32_t inner, float *__restrict__ out) {
@@ -330,9 +330,10 @@ int matmul_impl(yx_ctx *ctx, const float *x, const void *w_bf16, uint32_t T, uin
     if (tensor) {
         if (int rc = launch_matmul_tc(ctx, x, w, T, N, K, false, dst)) return rc;
     } else {
-        const uint64_t threads = (uint64_t)T * N * 32;
-        matmul_any_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, ctx->stream>>>(x, w, T, N, K, dst);
-        if (int rc = launched(ctx, "matmul kernel (any shape)")) return rc;
+        for (uint32_t t0 = 0; t0 < T; t0 += 65535u) {   // (the y extent's end)
+            matmul_any_kernel<<<dim3(N / 8 + 1, std::min(T - t0, 65535u)), 256, 0, ctx->stream>>>(x + (size_t)t0 * K, w, N, K, dst + (size_t)t0 * N);
+            if (int rc = launched(ctx, "matmul kernel (any shape)")) return rc;
+        }
     }
     if (!glu) return YX_OK;
     const uint64_t n = (uint64_t)T * cols;
