@@ -50,3 +50,15 @@ def test_gathers(backend, oracle, rows, h):
     assert np.array_equal(backend.to_host(e), want)
     sel = rng.integers(0, rows, rows)
     assert np.array_equal(backend.to_host(backend.select_rows(e, sel)), want[sel])
+
+
+@pytest.mark.parametrize("h", [65535 * 2048 + 8, 65535 * 2048 + 1])
+def test_gathers_of_rows_wider_than_a_grid(backend, h):
+    table = torch.arange(h, device=backend.device, dtype=torch.int32).remainder_(251).to(torch.bfloat16).view(1, h)
+    backend.begin_pass(PassMeta.from_rows([(0, 0)], [[0]]))
+    e = backend.embed(table)
+    backend.sync()
+    assert torch.equal(e, table.float())
+    del table
+    assert torch.equal(backend.select_rows(e, [0]), e)
+    backend.sync()

@@ -61,27 +61,31 @@ __device__ __forceinline__ void record_bad_row(yx_dev_status *status, int where,
 
 // out[r] = f32(table[ids[r]]) (cpu lib.rs:485-497); an id outside the table is recorded and its row zeroed.
 // Latency-bound at decode: a CTA takes 2048 columns of a row, eight to a thread in one 16-byte load where the
-// rows allow it (16 rows x 4096: 9.3 us with one scalar element at a time and a CTA per row).
+// rows allow it (16 rows x 4096: 9.3 us with one scalar element at a time and a CTA per row).  A grid's y extent ends
+// at 65535, so where a row has more parts than that a CTA takes several of them.
 constexpr uint32_t EMBED_COLS = 2048;
+dim3 gather_grid(uint32_t rows, uint32_t cols) { return dim3(rows, std::min((cols - 1) / EMBED_COLS + 1, 65535u)); }
 template <bool VEC>
 __global__ void __launch_bounds__(256) embed_kernel(const __nv_bfloat16 *__restrict__ table, uint32_t vocab, uint32_t h,
                                                     const __grid_constant__ RowIds ids, float *__restrict__ out, yx_dev_status *status) {
     dependent_entry();
-    const uint32_t r = blockIdx.x, id = ids.dev ? ids.dev[r] : ids.v[r], c0 = blockIdx.y * EMBED_COLS;
+    const uint32_t r = blockIdx.x, id = ids.dev ? ids.dev[r] : ids.v[r];
     const bool ok = id < vocab;
-    if (!ok && threadIdx.x == 0 && c0 == 0) record_bad_row(status, 400, id, r);
+    if (!ok && threadIdx.x == 0 && blockIdx.y == 0) record_bad_row(status, 400, id, r);
     const __nv_bfloat16 *src = table + (size_t)(ok ? id : 0u) * h;
     float *dst = out + (size_t)r * h;
-    if constexpr (VEC) {
-        const uint32_t c = c0 + threadIdx.x * 8;
-        if (c >= h) return;
-        const uint4 v = ok ? *(const uint4 *)(src + c) : make_uint4(0, 0, 0, 0);
-        auto lo = [](uint32_t w) { return __uint_as_float(w << 16); };
-        auto hi = [](uint32_t w) { return __uint_as_float(w & 0xffff0000u); };
-        *(float4 *)(dst + c) = make_float4(lo(v.x), hi(v.x), lo(v.y), hi(v.y));
-        *(float4 *)(dst + c + 4) = make_float4(lo(v.z), hi(v.z), lo(v.w), hi(v.w));
-    } else {
-        for (uint32_t c = c0 + threadIdx.x; c < min(h, c0 + EMBED_COLS); c += blockDim.x) dst[c] = ok ? __bfloat162float(src[c]) : 0.0f;
+    for (size_t c0 = (size_t)blockIdx.y * EMBED_COLS; c0 < h; c0 += (size_t)gridDim.y * EMBED_COLS) {
+        if constexpr (VEC) {
+            const size_t c = c0 + threadIdx.x * 8;
+            if (c >= h) return;
+            const uint4 v = ok ? *(const uint4 *)(src + c) : make_uint4(0, 0, 0, 0);
+            auto lo = [](uint32_t w) { return __uint_as_float(w << 16); };
+            auto hi = [](uint32_t w) { return __uint_as_float(w & 0xffff0000u); };
+            *(float4 *)(dst + c) = make_float4(lo(v.x), hi(v.x), lo(v.y), hi(v.y));
+            *(float4 *)(dst + c + 4) = make_float4(lo(v.z), hi(v.z), lo(v.w), hi(v.w));
+        } else {
+            for (size_t c = c0 + threadIdx.x; c < min((size_t)h, c0 + EMBED_COLS); c += blockDim.x) dst[c] = ok ? __bfloat162float(src[c]) : 0.0f;
+        }
     }
 }
 
@@ -90,22 +94,24 @@ __global__ void __launch_bounds__(256) select_rows_kernel(const float *__restric
                                                           const __grid_constant__ RowIds ids, float *__restrict__ out,
                                                           yx_dev_status *status) {
     dependent_entry();
-    const uint32_t r = blockIdx.x, src = ids.dev ? ids.dev[r] : ids.v[r], c0 = blockIdx.y * EMBED_COLS;
+    const uint32_t r = blockIdx.x, src = ids.dev ? ids.dev[r] : ids.v[r];
     if (src >= src_rows) {
-        if (threadIdx.x == 0 && c0 == 0) record_bad_row(status, 401, src, r);
+        if (threadIdx.x == 0 && blockIdx.y == 0) record_bad_row(status, 401, src, r);
         return;
     }
     const float *s = x + (size_t)src * cols;
     float *d = out + (size_t)r * cols;
-    const uint32_t end = min(cols, c0 + EMBED_COLS);
-    if constexpr (VEC) {
+    for (size_t c0 = (size_t)blockIdx.y * EMBED_COLS; c0 < cols; c0 += (size_t)gridDim.y * EMBED_COLS) {
+        const size_t end = min((size_t)cols, c0 + EMBED_COLS);
+        if constexpr (VEC) {
 #pragma unroll
-        for (uint32_t i = 0; i < EMBED_COLS / 1024; i++) {
-            const uint32_t c = c0 + i * 1024 + threadIdx.x * 4;
-            if (c < end) *(float4 *)(d + c) = *(const float4 *)(s + c);
+            for (uint32_t i = 0; i < EMBED_COLS / 1024; i++) {
+                const size_t c = c0 + i * 1024 + threadIdx.x * 4;
+                if (c < end) *(float4 *)(d + c) = *(const float4 *)(s + c);
+            }
+        } else {
+            for (size_t c = c0 + threadIdx.x; c < end; c += blockDim.x) d[c] = s[c];
         }
-    } else {
-        for (uint32_t c = c0 + threadIdx.x; c < end; c += blockDim.x) d[c] = s[c];
     }
 }
 
@@ -422,7 +428,7 @@ int yx_embed(yx_ctx *ctx, const void *table_bf16_dev, uint32_t vocab, uint32_t h
     const bool vec = h % 8 == 0 && (((uintptr_t)table_bf16_dev | (uintptr_t)out_dev) & 15u) == 0;
     ctx->last_launch = yx_ctx::LAST_OTHER;
     return launch_dependent(ctx, "embed kernel launch", vec ? embed_kernel<true> : embed_kernel<false>,
-                            dim3(rows, (h + EMBED_COLS - 1) / EMBED_COLS), dim3(256), 0, (const __nv_bfloat16 *)table_bf16_dev, vocab, h, ids,
+                            gather_grid(rows, h), dim3(256), 0, (const __nv_bfloat16 *)table_bf16_dev, vocab, h, ids,
                             out_dev, ctx->dev_status);
 }
 
@@ -439,7 +445,7 @@ int yx_select_rows(yx_ctx *ctx, const float *x_dev, uint32_t src_rows, uint32_t 
     const bool vec = cols % 4 == 0 && (((uintptr_t)x_dev | (uintptr_t)out_dev) & 15u) == 0;
     ctx->last_launch = yx_ctx::LAST_OTHER;
     return launch_dependent(ctx, "select_rows kernel launch", vec ? select_rows_kernel<true> : select_rows_kernel<false>,
-                            dim3(n, (cols + EMBED_COLS - 1) / EMBED_COLS), dim3(256), 0, x_dev, src_rows, cols, ids, out_dev,
+                            gather_grid(n, cols), dim3(256), 0, x_dev, src_rows, cols, ids, out_dev,
                             ctx->dev_status);
 }
 
