@@ -8,8 +8,8 @@
 use std::{env, path::PathBuf, process::Command};
 
 const SOURCES: &[&str] = &[
-    "api.cu", "kv_ops.cu", "attend_simt.cu", "attend_mma.cu", "prefill_tc.cu", "combine.cu", "dist.cu",
-    "attend_static.cu", "planner.cpp", "hooks.cu",
+    "api.cu", "kv_ops.cu", "attend_simt.cu", "attend_f32.cu", "attend_mma.cu", "prefill_tc.cu", "combine.cu", "dist.cu",
+    "attend_static.cu", "model_ops.cu", "matmul_tc.cu", "planner.cpp", "hooks.cu",
 ];
 
 fn main() {

@@ -57,6 +57,14 @@ def test_rust_ffi_block_matches_the_header():
         assert re.findall(r"pub (\w+):", body) == [f[0] for f in fields], c_name
 
 
+def test_the_crate_builds_what_the_library_is_built_from():
+    from yaxus_b200 import build
+    text = open(os.path.join(ROOT, "crates", "yaxus-backend-cuda", "build.rs")).read()
+    listed = text[text.index("const SOURCES"):]
+    assert sorted(re.findall(r'"([\w.]+)"', listed[:listed.index("];")])) == sorted(build.CUDA_SOURCES)
+    assert all(os.path.exists(os.path.join(build.CSRC, s)) for s in build.CUDA_SOURCES)
+
+
 def test_struct_sizes():
     assert ctypes.sizeof(_lib.Rope) == 65 * 4
     assert ctypes.sizeof(_lib.Layer) == 66 * 4
