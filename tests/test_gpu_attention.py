@@ -359,3 +359,31 @@ def test_lse_combine_of_strided_parts(backend):
     got = backend.lse_combine(m.T, l.T, o.transpose(0, 1))
     want = backend.lse_combine(m.T.contiguous(), l.T.contiguous(), o.transpose(0, 1).contiguous())
     assert torch.equal(got, want)
+
+
+def test_lse_combine_keeps_what_is_not_a_number(backend):
+    # element 0: every part sound; 1: one part's sum is no number, as a key of score NaN leaves it; 2: one part empty, its vector unwritten
+    m, l, o = torch.zeros(3, 3), torch.ones(3, 3), torch.ones(3, 3, 128)
+    l[1, 1], l[2, 2], m[2, 2], o[2, 2] = float("nan"), 0.0, -1e30, float("nan")
+    got = backend.to_host(backend.lse_combine(dev(backend, m), dev(backend, l), dev(backend, o)))
+    assert (got[0] == 1).all() and np.isnan(got[1]).all() and (got[2] == 1).all()
+
+
+@pytest.mark.parametrize("merge", ["kernel", "fused", "static"])
+def test_a_key_without_a_score_shows_in_16_bits(backend, merge):
+    s = W.build("no-score", 22, 16, 4, F16, [1500, 900], [1, 1])
+    page, at = divmod(700, 128)
+    s.k_bits[int(s.tables[0][page]) * 128 + at] = np.float16(np.nan).view(np.uint16)
+    kv = load(backend, s)
+    backend.begin_pass(s.meta)
+    backend.kv_append(kv, 0, dev(backend, s.k_new), dev(backend, s.v_new))
+    q, out = dev(backend, s.q), torch.zeros(2, s.hq * 128, device=backend.device)
+    if merge == "static":
+        assert backend._L.yx_attend_static(backend._ctx, kv._h, 0, q.data_ptr(), F32, s.hq, -1, out.data_ptr(), F32) == 0
+    else:
+        backend.set_tuning(fused_merge=merge == "fused")
+        backend.attend(kv, 0, q, s.hq, out=out)
+        backend.set_tuning()
+    got = backend.to_host(out)
+    assert not np.isfinite(got[0]).any() and np.isfinite(got[1]).all()
+    kv.close()

@@ -512,7 +512,7 @@ __device__ __forceinline__ void merge_completed(const Epilogue &E, const uint32_
 #pragma unroll 2
             for (uint32_t c = 0; c < nc; c++) {
                 const float2 v = mls[c];
-                if (!(v.y > 0.0f)) continue;
+                if (v.y <= 0.0f) continue;   // (empty; a sum that is no number shows in the row)
                 const float w = __expf(v.x - mx);
                 ls += v.y * w;
                 const float4 *src = (const float4 *)(po + (size_t)(c0 + c) * group * D);

@@ -215,13 +215,13 @@ attend_static_merge_kernel(const StaticScratch *__restrict__ scratch, int hq, in
     for (int s = 0; s < SPLITS; s++) {
         const size_t slot = first + (size_t)s * group;
         const float el = scratch->ml[slot * 2 + 1];
-        if (el > 0.0f) {
+        if (!(el <= 0.0f)) {   // (a sum that is no number shows in the row)
             const float w = exp2f((scratch->ml[slot * 2] - mx) * LOG2E);
             l += el * w;
             acc += scratch->o[slot * D + t] * w;
         }
     }
-    sm_out[t] = l > 0.0f ? acc / l : 0.0f;
+    sm_out[t] = l == 0.0f ? 0.0f : acc / l;
     __syncthreads();
     if (t < D / 4)
         dev::store4(out, out_dtype, ((size_t)row * hq + h) * D + t * 4,

@@ -143,7 +143,7 @@ __global__ void combine_flat_kernel(int n_parts, const float *__restrict__ m, co
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int c = 0; c < n_parts; c++) {
         float em = m[(size_t)c * sm + idx], el = l[(size_t)c * sl + idx];
-        if (!(el > 0.0f)) continue;
+        if (el <= 0.0f) continue;   // (empty; a sum that is no number shows in the result)
         float4 po = *(const float4 *)(o + (size_t)c * so + idx * D + lane * 4);
         float nm = fmaxf(mx, em);
         float r = __expf(mx - nm), w = __expf(em - nm);
