@@ -65,7 +65,7 @@ typedef struct yx_layer {
 /* Kernel choices, the counterpart of the reference's `Tuning`
  * (crates/yaxus-backend-gpu/src/device.rs:96-167).  Zero means "library default". */
 typedef struct yx_tuning {
-    int32_t force_path;      /* 0 auto, 1 SIMT split-key, 2 tensor split-key, 3 tcgen05 tiles */
+    int32_t force_path;      /* 0 auto, 1 SIMT split-key, 2 tensor split-key, 3 tcgen05 tiles (f32 caches: SIMT tiles) */
     int32_t ctas_per_sm;     /* persistent CTAs per SM for the split-key kernels (0: default, 4 for the SIMT kernel and
                                 for the tensor kernel one per SM with one SM left spare for the call behind) */
     int32_t share_prefix;    /* 0 default (on), 1 on, 2 off: read pages shared by several rows once */

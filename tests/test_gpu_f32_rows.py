@@ -10,8 +10,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("bad", [np.nan, np.inf])
-@pytest.mark.parametrize("ctx,rows,launches", [(40, 1, 1), (1500, 1, 1), (1500, 40, 2)])   # one part, many parts; the tiled kernel and its merge
-def test_a_key_without_a_score_shows(backend, oracle, bad, ctx, rows, launches):
+@pytest.mark.parametrize("ctx,rows,kernel", [(40, 1, 1), (1500, 1, 1), (1500, 40, 3)])   # one part, many parts; the tiled kernel and its merge
+def test_a_key_without_a_score_shows(backend, oracle, bad, ctx, rows, kernel):
     """Every row that sees a key of score NaN or +inf comes out as no number, however its keys are cut; others are untouched."""
     s = W.build("f32-no-score", 21, 16, 4, F32, [ctx, 900], [rows, rows])
     s.q[:, ::128] = np.abs(s.q[:, ::128]) + 0.1          # (dim 0 of every head: a score of +inf, never -inf)
@@ -22,11 +22,13 @@ def test_a_key_without_a_score_shows(backend, oracle, bad, ctx, rows, launches):
     backend.begin_pass(s.meta)
     backend.kv_append(kv, 0, dev(backend, s.k_new), dev(backend, s.v_new))
     q = dev(backend, s.q)
+    backend.set_tuning(force_path=kernel)
     got = backend.to_host(backend.attend(kv, 0, q, s.hq)).reshape(2 * rows, s.hq, 128)
-    assert backend.last_plan().launches == launches
+    assert backend.last_plan().launches == (1 if kernel == 1 else 2)
     assert not np.isfinite(got[:rows]).any()
     assert_close(got[rows:].reshape(rows, -1), want[rows:], abs_tol=2e-5, rel_tol=0.0, what="the rows beside it")
     _, l, o = (backend.to_host(t) for t in backend.attend_partial(kv, 0, q, s.hq, None, 0, 1 << 40))
+    backend.set_tuning()
     assert not np.isfinite(l[:rows]).any()
     assert_close(o[rows:] / l[rows:, :, None], got[rows:], abs_tol=2e-5, rel_tol=0.0, what="triples of the rows beside it")
     kv.close()

@@ -257,6 +257,36 @@ int pick_path(const yx_ctx *ctx, const yx_kv *kv) {
     return 2;
 }
 
+// Which of the two f32 kernels a pass is quicker with, by what each was measured to take (nanoseconds; 1 to 32 sequences
+// of 0 to 20000 keys, 1 to 1000 rows each, 1 to 16 query heads a KV head).  A row costs the row kernel 0.18 a key, KV head
+// and four query heads (which it takes one sweep after the other), and as much as 80 keys by itself; a unit of up to 16, 32
+// or 64 queries costs the tiled one 0.60, 0.72 or 1.2 a key and KV head.  A unit's tile is the longer chain of latencies
+// and the merge a launch: that is what a pass of few keys pays, as every sweep after the first is on the other side.  16
+// query / 4 KV heads, us by rows and by tiles: twelve sequences of 600 to 2500 keys, one row each 25 and 56, one of them
+// with five rows 31 and 56, with 40 rows 55 and 71, with 100 rows 116 and 96; five rows each 74 and 63; one of 1000 keys with
+// 16 rows 19 and 31, with 64 rows 55 and 41.  Of 270 such passes the rule gives three more than a tenth away, 19 % at most.
+bool f32_tiles_pay(const PassHost &p, int group, int hkv, int64_t window, uint64_t key_lo, uint64_t key_hi) {
+    const uint32_t unit_rows = (uint32_t)std::max(1, std::min(MAX_ITEM_ROWS, 64 / group));
+    const int sweeps = (group + 3) / 4;
+    float by_rows = 6500.0f * (float)(sweeps - 1), by_tiles = 0.0f, chain = 0.0f;
+    for (const PassHost::Run &run : p.runs) {
+        uint64_t seen = run.keys / run.rows;   // keys a row sees, on average
+        if (window > 0) seen = std::min(seen, (uint64_t)window);
+        seen = std::min(seen, key_hi - std::min(key_lo, key_hi));
+        const float keys = (float)seen * (float)hkv;
+        by_rows += 0.18f * (float)sweeps * (float)run.rows * (keys + 80.0f * (float)hkv);
+        auto units = [&](uint32_t n, uint32_t rows) {
+            const uint32_t queries = n > 0 ? rows * (uint32_t)group : 0;
+            if (queries == 0) return;
+            by_tiles += (queries <= 16 ? 0.60f : queries <= 32 ? 0.72f : 1.2f) * (float)n * keys;
+            chain = std::max(chain, queries <= 16 ? 5000.0f : queries <= 32 ? 6000.0f : 19000.0f);
+        };
+        units(run.rows / unit_rows, unit_rows);
+        units(1, run.rows % unit_rows);
+    }
+    return by_tiles + chain < by_rows;
+}
+
 // What yx_attention does to the step's rows before it attends: norm, RoPE, append, queries to `q`.
 struct RopeAppend {
     const float *qkv, *q_norm, *k_norm;
@@ -285,10 +315,9 @@ int attend_impl(yx_ctx *ctx, yx_kv *kv, int layer, const void *q, int q_dtype, i
     DeviceGuard guard(ctx->device);
 
     const int path = pick_path(ctx, kv);
-    // f32 caches: where some sequence brings more than 16 queries to a KV head, tiles of keys shared by up to 64 of them.
-    // One row a sequence is better off with the kernel that takes a row at a time (12 sequences of 600 to 2500 keys, two
-    // layers: 108 us there, 125 us here), and asking for path 1 gets that kernel.
-    const bool f32_tiles = path == 1 && kv->dtype == YX_F32 && ctx->tuning.force_path != 1 && (uint64_t)ctx->pass.longest_run * group > 16;
+    // f32 caches: a row at a time, or tiles of keys shared by up to 64 queries; asking for path 1 or 3 gets one or the other.
+    const bool f32_tiles = path == 1 && kv->dtype == YX_F32 && ctx->tuning.force_path != 1 &&
+                           (ctx->tuning.force_path == 3 || f32_tiles_pay(ctx->pass, group, kv->hkv, window, key_lo, key_hi));
     const int64_t launches0 = ctx->launches;
     PlanParams pp{};
     pp.hkv = kv->hkv;
@@ -781,15 +810,13 @@ int yx_begin_pass(yx_ctx *ctx, uint32_t rows, const uint32_t *pos, const uint32_
     if (rows && (!pos || !kv_slot || !pt_off)) return fail(ctx, YX_ERR_INVALID, "begin_pass: null array");
     if (n_pages && !pages) return fail(ctx, YX_ERR_INVALID, "begin_pass: null page table");
     if (rows > 65535) return fail(ctx, YX_ERR_UNSUPPORTED, "begin_pass: more than 65535 rows");
-    uint32_t max_pos = 0, max_slot = 0, max_page = 0, run = 0, longest_run = 0;
+    uint32_t max_pos = 0, max_slot = 0, max_page = 0;
     for (uint32_t r = 0; r < rows; r++) {
         if ((uint64_t)pt_off[r] + pos[r] / PAGE >= n_pages)
             return fail(ctx, YX_ERR_INVALID, "begin_pass: a row's page table runs past `pages`");
         // kv_slot must be the slot of the row's own position (PassMeta, lib.rs:69-70).
         if (kv_slot[r] != pages[pt_off[r] + pos[r] / PAGE] * (uint32_t)PAGE + pos[r] % PAGE)
             return fail(ctx, YX_ERR_INVALID, "begin_pass: kv_slot is not slot(pages, pos)");
-        run = r > 0 && pt_off[r] == pt_off[r - 1] ? run + 1 : 1;
-        longest_run = std::max(longest_run, run);
         max_pos = std::max(max_pos, pos[r]);
         max_slot = std::max(max_slot, kv_slot[r]);
     }
@@ -804,7 +831,12 @@ int yx_begin_pass(yx_ctx *ctx, uint32_t rows, const uint32_t *pos, const uint32_
     p.max_pos_seen = max_pos;
     p.max_slot_seen = max_slot;
     p.max_page_seen = max_page;
-    p.longest_run = longest_run;
+    p.runs.clear();
+    for (uint32_t r = 0; r < rows; r++) {
+        if (r == 0 || pt_off[r] != pt_off[r - 1]) p.runs.push_back({0, 0});
+        p.runs.back().rows++;
+        p.runs.back().keys += (uint64_t)pos[r] + 1;
+    }
     ctx->pass_serial++;
     ctx->have_pass = true;
 

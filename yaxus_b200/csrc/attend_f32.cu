@@ -4,6 +4,7 @@
 // (rows, one KV head, a run of keys) the running maximum m, the sum of exponentials l and the unnormalised
 // output o of every query head of the KV head's group.
 //
+// For passes that bring enough queries to the same keys (api.cu, f32_tiles_pay, says which those are).
 // An item brings up to 64 queries (rows x heads of the group) to the same keys, and a tile of 32 keys is used for
 // all of them out of shared memory: with one row an item, a prompt of 1000 rows read every key 1000 times and was
 // bound by the shuffles of its dot products.  128 threads, two CTAs an SM: thread (ty, tx) of 8 x 16 holds rows
@@ -14,7 +15,7 @@
 // them there, two tiles in flight.
 //
 // Bound by the latencies of its own arithmetic at two warps a scheduler (FMA pipe half busy), not by memory.  A
-// 1000-row prompt behind 1000 keys, 16 query / 4 KV heads, two layers: a whole step 5415 -> 1385 us.
+// 1000-row prompt behind 1000 keys, 16 query / 4 KV heads, two layers: a whole step 5415 -> 1340 us.
 // Sums are blocked by 32 dims and 32 keys, which costs 36 us of that: the error against 64 bits over 300 rows behind
 // 1000 keys is 2.0e-7 with it, 4.0e-7 without, and 3.3e-7 for the kernel that takes a row at a time.
 #include <type_traits>

@@ -182,7 +182,11 @@ struct PassHost {
     uint32_t max_pos_seen = 0;    // largest position of a row
     uint32_t max_page_seen = 0;   // largest page id in `pages`
     uint32_t max_slot_seen = 0;   // largest kv_slot of a row
-    uint32_t longest_run = 0;     // most rows in a row with one page table
+    struct Run {
+        uint32_t rows;            // rows in a row with one page table
+        uint64_t keys;            // the keys up to each of them, added up
+    };
+    std::vector<Run> runs;
 };
 
 struct PlanParams {
