@@ -64,7 +64,6 @@ struct TileParams {
     int out_dtype;
     int bf16;            // cache type: 1 bf16, 0 f16
     int q_lo;            // queries carry a low part (f32 queries on a bf16 cache): S = Qh K^T + Ql K^T
-    int p_lo;            // probabilities carry a low part (bf16 cache): O += Ph V + Pl V
     yx_dev_status *status;
     long long *trace;   // diagnostics: clock stamps of CTA 0's pipeline, or null
     const uint32_t *cta_begin;   // items of persistent CTA c: [cta_begin[c], cta_begin[c + 1])
@@ -347,7 +346,10 @@ __global__ void __launch_bounds__(THREADS, 1) prefill_tc_kernel(const TileParams
             for (int i = 0; i < 64; i++) mxs[i & 3] = fmaxf(mxs[i & 3], __uint_as_float(sr[i >> 5][i & 31]));
             float mx = fmaxf(fmaxf(mxs[0], mxs[1]), fmaxf(mxs[2], mxs[3]));
             row_part[b][half][r] = mx;
+            // (each half's probabilities go over columns that the other half's scores were read from: their loads come first)
+            tc_fence_before();
             asm volatile("bar.sync 1, %0;" ::"n"(SOFTMAX_WARPS * 32) : "memory");
+            tc_fence_after();
             mx = fmaxf(mx, row_part[b][half ^ 1][r]);
             // Lazy rescaling: keep the old reference maximum while the new one is within 2^8.
             float alpha = 1.f;
@@ -1054,7 +1056,6 @@ int launch_prefill_tc(yx_ctx *ctx, const TileArgs &a) {
     P.out = a.out;
     P.out_dtype = a.out_dtype;
     P.bf16 = a.kv_dtype == YX_BF16 ? 1 : 0;
-    P.p_lo = P.bf16;
     P.q_lo = P.bf16 && a.q_dtype == YX_F32;
     P.status = ctx->dev_status;
     P.trace = (long long *)ctx->trace_buf;
