@@ -46,7 +46,8 @@ def test_matmul_tiles(backend, oracle, t, n, k):
 
 @pytest.mark.parametrize("t,inner,k", [
     (1, 16, 128), (8, 1040, 256), (13, 48, 1024), (32, 9696, 128), (5, 24, 256),
-    (33, 16, 128), (48, 144, 1024), (257, 1040, 256), (100, 24, 256), (150, 9696, 128), (35, 9696, 128), (60, 19456, 128)])
+    (33, 16, 128), (48, 144, 1024), (257, 1040, 256), (100, 24, 256), (150, 9696, 128), (35, 9696, 128), (60, 19456, 128),
+    (300, 9696, 256)])                                      # two tiles of pass rows, two whole rounds of tiles and a remainder
 def test_glu_tiles(backend, oracle, t, inner, k):
     x, w_bits = inputs(oracle, t, 2 * inner, k)
     w = backend.load_weight(w_bits)
@@ -61,6 +62,20 @@ def test_glu_tiles(backend, oracle, t, inner, k):
     assert np.array_equal(backend.to_host(backend.matmul_glu(xd, w)), got)
 
 
+@pytest.mark.parametrize("t,n,k", [(170, 18944, 3072), (512, 9700, 6016)])   # 18 and 32 steps, the most
+def test_a_longer_first_chain(backend, t, n, k):
+    # more than 160 rows a tile (two accumulators) and whole tiles of 48 and 94 k steps: a piece begins with a longer chain
+    gen = torch.Generator(device=backend.device)
+    gen.manual_seed(k)
+    x = torch.randn(t, k, generator=gen, device=backend.device)
+    w = (torch.randn(n, k, generator=gen, device=backend.device) * k ** -0.5).bfloat16()
+    got = backend.matmul(x, w)
+    backend.sync()
+    xd, wd = x.double(), w.double().T
+    # an accumulator is added to up to 256 times (32 steps, four of 16 k in each, two parts) and may drop its last place each time
+    assert ((got - xd @ wd).abs() <= (2.0 ** -17 + 256 * 2.0 ** -23) * (xd.abs() @ wd.abs())).all()
+
+
 @pytest.mark.parametrize("t", [5, 70])
 def test_unaligned_rows(backend, oracle, t):
     # pass rows that start 8 bytes past a 16-byte boundary
@@ -70,6 +85,21 @@ def test_unaligned_rows(backend, oracle, t):
     xd.copy_(torch.from_numpy(x))
     got = backend.to_host(backend.matmul(xd, backend.load_weight(w_bits)))
     assert (np.abs(got - oracle.matmul(x, w_bits)) <= TOL * magnitudes(x, w_bits)).all()
+
+
+@pytest.mark.parametrize("t,n,glu", [(1, 60000, 0), (1, 60000, 1), (32, 4096, 0), (70, 4096, 0), (70, 8192, 1)])
+def test_a_result_over_its_own_rows(backend, t, n, glu):
+    k = 4096
+    gen = torch.Generator(device=backend.device)
+    gen.manual_seed(t)
+    x, w = torch.randn(t, k, generator=gen, device=backend.device), torch.randn(n, k, generator=gen, device=backend.device).mul_(k ** -0.5).bfloat16()
+    want = (backend.matmul_glu if glu else backend.matmul)(x, w)
+    both = torch.zeros_like(want)
+    both.view(-1)[:t * k] = x.view(-1)
+    call = backend._L.yx_matmul_glu if glu else backend._L.yx_matmul
+    assert call(backend._ctx, both.data_ptr(), w.data_ptr(), t, n, k, both.data_ptr()) == 0
+    backend.sync()
+    assert torch.equal(both, want)
 
 
 def test_more_outputs_than_a_32_bit_thread_index_reaches(backend):

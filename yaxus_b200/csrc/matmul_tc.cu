@@ -165,7 +165,8 @@ __device__ __forceinline__ void store_rows(const PairArgs &a, const float (&v)[3
 }
 
 // CHUNKS: 64-row chunks of a tile, what an epilogue thread keeps in registers (two for up to
-// 128 pass rows, three for up to 192: steps of 80 and of 311 rows take 391 and 453 us with room for four, 382 and 437 so).
+// 128 pass rows, three for up to 192: before the chains of eight above, steps of 80 and of 311 rows took 391 and 453 us with
+// room for four, 382 and 437 so; with them 399 and 440).
 template <bool GLU, int CHUNKS>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
 matmul_pair_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap x_map, const PairArgs a) {
@@ -865,6 +866,14 @@ int matmul_few_rows(yx_ctx *ctx, const float *x, const void *w, uint32_t T, uint
         configured = true;
     }
     RowsArgs a{};
+    // Other CTAs still read the rows when a tile's result is written: a result over its own rows takes them from a copy.
+    const uintptr_t x0 = (uintptr_t)x, o0 = (uintptr_t)out;
+    if (o0 < x0 + (size_t)T * K * 4 && x0 < o0 + (size_t)T * (GLU ? N / 2 : N) * 4) {
+        if (int rc = ensure_buffer(ctx, (void **)&ctx->mm_packed, &ctx->mm_packed_cap, (size_t)ROWS_MAX * K * 4)) return rc;
+        if (int rc = check_cuda(ctx, cudaMemcpyAsync(ctx->mm_packed, x, (size_t)T * K * 4, cudaMemcpyDeviceToDevice, ctx->stream), "matmul: rows under the result"))
+            return rc;
+        x = (const float *)ctx->mm_packed;
+    }
     a.x = x;
     a.T = T;
     a.K = K;
@@ -901,7 +910,7 @@ int matmul_tc(yx_ctx *ctx, const float *x, const void *w, uint32_t T, uint32_t N
 
 }  // namespace
 
-// Takes K a multiple of 64, w 16-byte aligned, x 8-byte aligned; with `glu`, a multiple of 16 result columns.
+// Takes K a multiple of 128, w 16-byte aligned, x 8-byte aligned; with `glu`, a multiple of 16 result columns.
 int launch_matmul_tc(yx_ctx *ctx, const float *x, const void *w, uint32_t T, uint32_t N, uint32_t K, bool glu, float *out) {
     return glu ? matmul_tc<true>(ctx, x, w, T, N, K, out) : matmul_tc<false>(ctx, x, w, T, N, K, out);
 }
