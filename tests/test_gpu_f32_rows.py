@@ -1,10 +1,11 @@
 """Attention over f32 caches a row at a time: parts of a row whose sums are no numbers."""
 import numpy as np
 import pytest
+import torch
 
 from oracle.check import assert_close, dev, load, oracle_step
 from yaxus_b200 import workloads as W
-from yaxus_b200._lib import F32
+from yaxus_b200._lib import F16, F32
 
 pytestmark = pytest.mark.gpu
 
@@ -31,4 +32,20 @@ def test_a_key_without_a_score_shows(backend, oracle, bad, ctx, rows, kernel):
     backend.set_tuning()
     assert not np.isfinite(l[:rows]).any()
     assert_close(o[rows:] / l[rows:, :, None], got[rows:], abs_tol=2e-5, rel_tol=0.0, what="triples of the rows beside it")
+    kv.close()
+
+
+@pytest.mark.parametrize("dtype", [F32, F16])
+def test_a_result_over_its_queries(backend, dtype):
+    # A row of 16-bit results lies over the queries of a row half as far up.
+    s = W.build("f32-over", 23, 16, 4, F32, [2500] * 32 + [10] * 32, [1] * 64)
+    kv = load(backend, s)
+    backend.begin_pass(s.meta)
+    backend.kv_append(kv, 0, dev(backend, s.k_new), dev(backend, s.v_new))
+    q = dev(backend, s.q)
+    want = backend.attend(kv, 0, q, s.hq, out_dtype=torch.float32 if dtype == F32 else torch.float16)
+    assert backend.last_plan().launches == 1
+    assert backend._L.yx_attend(backend._ctx, kv._h, 0, q.data_ptr(), F32, s.hq, -1, q.data_ptr(), dtype) == 0
+    backend.sync()
+    assert torch.equal(q.view(-1).view(want.dtype)[:want.numel()], want.view(-1))
     kv.close()

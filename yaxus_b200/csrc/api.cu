@@ -387,6 +387,21 @@ int attend_impl(yx_ctx *ctx, yx_kv *kv, int layer, const void *q, int q_dtype, i
         }
     }
 
+    // The row kernel writes a row as soon as its last part is in, while others' queries are still read: results over other
+    // rows' queries, which a merge behind the kernel would leave unharmed, take the queries from a copy.
+    if (path == 1 && !f32_tiles) {
+        const size_t n = (size_t)ctx->pass.rows * hq, q_size = q_dtype == YX_F32 ? 4 : 2, q_bytes = n * D * q_size;
+        auto over = [&](const void *p, size_t bytes) { return p && (uintptr_t)p < (uintptr_t)q + q_bytes && (uintptr_t)q < (uintptr_t)p + bytes; };
+        const size_t out_size = out_dtype == YX_F32 ? 4 : 2;
+        const bool own_rows_only = (out == q && out_size == q_size) || (o_out == q && q_size == 4);   // (a row and KV head's queries have all been read by then)
+        if ((!own_rows_only && (over(out, n * D * out_size) || over(o_out, n * D * 4))) || over(m_out, n * 4) || over(l_out, n * 4)) {
+            if (int rc = ensure_buffer(ctx, (void **)&ctx->q_tmp, &ctx->q_tmp_cap, q_bytes)) return rc;
+            if (int rc = check_cuda(ctx, cudaMemcpyAsync(ctx->q_tmp, q, q_bytes, cudaMemcpyDeviceToDevice, ctx->stream), "attend: queries under the result"))
+                return rc;
+            q = ctx->q_tmp;
+        }
+    }
+
     bool early_kv = predecessor_wrote_marked_tiles_only;
     if (pre) {
         // write_rows, then attend (cpu lib.rs:526-529): all rows' K/V land before any row attends.
