@@ -126,11 +126,7 @@ attend_simt_kernel(const void *__restrict__ q, int q_dtype, int hq, int group, c
     __shared__ bool last;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const float scale = 0.08838834764831845f;   // 1 / sqrt(128), the reference's f32 value
-    // A programmatic dependent of the kernel before it: resident while that kernel finishes, it
-    // waits here for everything earlier to be complete, and only then lets the merge kernel behind
-    // it become resident in turn.
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    dev::dependent_entry();
     const uint32_t ib = cta_begin[blockIdx.x], ie = cta_begin[blockIdx.x + 1];
     for (uint32_t ii = ib; ii < ie; ii++) {
         const Item it = items[ii];
