@@ -45,14 +45,19 @@ constexpr int TC_TMA_WARP = 8, TC_MMA_WARP = 9;
 constexpr uint32_t W_BYTES = 128 * 128;     // a CTA's share of a stage's weights
 constexpr uint32_t TC_SMEM_BUDGET = 220 * 1024;
 // k steps summed in tensor memory before the epilogue takes them over into its own f32 sums: the tensor core drops what
-// lies below its accumulator's last place (see ROWS_CHAIN below).  Error of the result against 64-bit products, 512 rows
-// x [28672, 4096] with a GLU: one chain 1.9e-5, two library products 0.97e-5, chains of 16 0.64e-5.  Tiles of up to 128
-// rows take chains of eight, without which 80 rows x [50257, 4096] lose against the library (8.5e-6 in one chain, 3.3e-6
-// in chains of 16, 2.7e-6 in chains of eight and in the library); a step of 80 rows pays 19 us of 399 for that.  Where
-// only two accumulators fit, a piece begins with a longer chain: it is what the tensor cores have to do while the
-// epilogue stores the piece before (2048 rows x [28672, 4096]: 608 us, with chains of eight throughout 665, without
-// chains 590).
-constexpr uint32_t TC_CHAIN = 16, TC_FIRST_CHAIN = 32;
+// lies below its accumulator's last place at each of a step's eight additions (see ROWS_CHAIN below).  Whole rounds of tiles of
+// more than 128 rows and 32 k steps or more take chains of 16.  Error of the result against 64-bit products, 512 rows x
+// [28672, 4096] with a GLU: one chain 1.9e-5, two library products 0.97e-5, chains of 16 0.64e-5; there, a piece begins with
+// a longer chain where only two accumulators fit: it is what the tensor cores have to do while the epilogue stores the
+// piece before (2048 rows x [28672, 4096]: 608 us, with chains of eight throughout 665, without chains 590).
+// Everything else takes chains that lose no more than two library products would, whose accumulators take half the
+// additions (one part each) and which cut k for small results: eight steps, half of the k steps where there are fewer than
+// 16 of them, six where every tile is cut along k.  Errors with chains of 16, now, and the library's (2.44e-6 of each is
+// the activations' two parts'): 275 rows x [34914, 1152] 3.19, 2.67 and 2.70e-6; 262 x [1460, 6784] 3.27, 2.60 and 2.60e-6;
+// 558 x [41408, 1024] with a GLU 5.70, 4.22 and 4.09e-6.  Over 110 shapes of 33 to 900 rows at most 1.05 times the
+// library's (1.39 before).  It costs 1 % in the mean, 6 % where it costs most (the last of these: 90 and 96 us); a step of
+// 80 rows pays 19 us of 399 for chains of eight in place of 16.
+constexpr uint32_t TC_CHAIN = 16, TC_FIRST_CHAIN = 32, TC_SHORT_CHAIN = 8, TC_CUT_CHAIN = 6, TC_LEAST_CHAIN = 4;
 constexpr int TC_MAX_BUFS = 4;
 constexpr uint32_t GLU_GROUP = 16;          // gate and up rows alternate in a tile sixteen by sixteen: a warp holds both
 
@@ -65,6 +70,7 @@ struct PairArgs {
     uint32_t rest_units, rest_pairs;  // k steps of the tiles after them, and the pairs that share those
     uint32_t stages;
     uint32_t bufs, buf_columns;       // accumulators in tensor memory
+    uint32_t chain, long_first;       // k steps summed in one of them; whether a piece begins with more
     float *out;
     float *part;                      // [2 * rest_pairs shares][2 CTAs][bt][128]
     uint32_t *counters;               // [tiles left over][2 CTAs], zero between launches
@@ -111,8 +117,7 @@ struct Walk {
 
 // Where the chain of k steps that begins at k ends.
 __device__ __forceinline__ uint32_t chain_end(const PairArgs &a, const Piece &p, uint32_t k) {
-    uint32_t n = a.bufs == TC_MAX_BUFS ? TC_CHAIN / 2 : TC_CHAIN;
-    if (k == p.k0 && a.bufs == 2) n = min(TC_FIRST_CHAIN, max(TC_CHAIN, (p.k1 - p.k0) * 3 / 8));
+    const uint32_t n = k == p.k0 && a.long_first ? min(TC_FIRST_CHAIN, max(a.chain, (p.k1 - p.k0) * 3 / 8)) : a.chain;
     return min(p.k1, k + n);
 }
 // Accumulators in turn, and the parity of the current round of them.
@@ -828,6 +833,9 @@ int matmul_pair_rows(yx_ctx *ctx, const float *x, const void *w, uint32_t T, uin
     a.stages = std::min<uint32_t>(TC_MAX_STAGES, (TC_SMEM_BUDGET - 1024) / stage_bytes);
     a.bufs = a.bt <= 128 ? 4 : a.bt <= 160 ? 3 : 2;
     a.buf_columns = 512 / a.bufs / 32 * 32;
+    const bool large = a.bufs < TC_MAX_BUFS && a.rounds > 0 && a.ksteps >= 2 * TC_CHAIN;
+    a.chain = large ? TC_CHAIN : std::min(a.rounds > 0 ? TC_SHORT_CHAIN : TC_CUT_CHAIN, std::max(TC_LEAST_CHAIN, a.ksteps / 2));
+    a.long_first = large && a.bufs == 2;
     a.out = out;
     a.status = ctx->dev_status;
     // The most any pass needs (39 MB), so that a call that is being recorded into a graph finds it whatever passes came
